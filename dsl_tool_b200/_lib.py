@@ -198,6 +198,7 @@ def scratch_word(device: torch.device) -> torch.Tensor:
 
 
 _workspace: Dict[tuple, torch.Tensor] = {}
+_retired_workspaces: list = []
 WORKSPACE_BYTES = 16 << 20
 
 
@@ -212,6 +213,11 @@ def workspace(device: torch.device, need: int = WORKSPACE_BYTES) -> Optional[tor
     key = (idx, torch.cuda.current_stream(device).cuda_stream)
     t = _workspace.get(key)
     if t is None or t.numel() < need:
+        if torch.cuda.is_current_stream_capturing():
+            # memory allocated under capture belongs to that graph's pool: the caller holds it for this call only
+            return torch.empty(int(need), dtype=torch.uint8, device=device)
+        if t is not None:
+            _retired_workspaces.append(t)      # a captured CUDA graph may still point at it
         t = torch.empty(max(int(need), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
         _workspace[key] = t
     return t

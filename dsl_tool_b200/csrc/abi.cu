@@ -211,7 +211,8 @@ size_t dsl_workspace_bytes(int op, long long M, int N, int K, int groups) {
         case DSL_OP_GEMM_BF16: kind = KIND_BF16; k_bytes = 2ll * K; break;
         case DSL_OP_GEMM_FP4_NV: kind = KIND_NVF4; k_bytes = K / 2; break;
         case DSL_OP_GEMM_FP4_MX: kind = KIND_MXF4; k_bytes = K / 2; break;
-        default: return 0;                            // the group-scaled FP8 GEMM and the quantisers use none
+        case DSL_OP_GEMM_FP8_GROUPWISE: kind = KIND_F8G; k_bytes = K; break;
+        default: return 0;                            // the quantisers use none
     }
     if (k_bytes <= 0 || k_bytes > 0x7FFFFFFFll) return 0;
     GemmArgs a{};

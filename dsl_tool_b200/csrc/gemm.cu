@@ -513,6 +513,7 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args) {
         const size_t b = decode_scratch_bytes(kind, args, &served);
         if (served) return b > 0 ? b + DSL_WS_HEADER_BYTES : 0;
     }
+    if (kind == KIND_F8G) return 0;      // its tiled kernels never split K
     if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) return 0;
     long long max_tiles = 0;
     one_cta_tiles(args, &max_tiles);

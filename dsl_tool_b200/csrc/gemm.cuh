@@ -10,7 +10,7 @@
 
 namespace dsl {
 
-enum { KIND_F8 = 0, KIND_NVF4 = 1, KIND_MXF4 = 2, KIND_BF16 = 3 };
+enum { KIND_F8 = 0, KIND_NVF4 = 1, KIND_MXF4 = 2, KIND_BF16 = 3, KIND_F8G = 4 /* FP8 with fp32 scales per 128 K */ };
 
 struct GemmArgs {
     int m_total;                 // rows of A / C over all row groups

@@ -19,6 +19,12 @@
 //     ever stores anything else, carry a per-launch epoch (a word of another epoch counts as empty) and
 //     are zeroed by the CTA that finishes the tile, so scratch needs no initialisation.  Both ways the
 //     result is identical from run to run.
+//   * Group-scaled FP8 (fp32 scales per 128 K, KIND_F8G) streams the same way, but every K group's partial product passes
+//     through registers (promote_run): one TOK-column buffer of tensor memory per stage in a ring of 4 or 8, four
+//     multiply-add warps.  Its tiled kernels compute 128 x 256 tiles whatever the row count, i.e. 16 busy SMs for 4096
+//     columns: 16 x 4096 x 14336 with 128x128 block scales took 73.0 us per call (quantiser included), 19.6 us here,
+//     the kernel alone 16.1 us = 3.6 TB/s of weight.  Bound by the weight stream plus about 7 us of launch, first bytes
+//     and combine, as for the other kinds.
 //   * The kernel is launched with programmatic stream serialisation: set-up, and for a weight
 //     the caller declares static also the first ring of weight tiles, overlap the tail of the
 //     preceding kernel (the activation quantiser); everything else waits for it.
@@ -64,10 +70,16 @@ struct DecCfg {
     static constexpr int OFF_SFX = OFF_SFW + NUM_STAGES * SF_STAGE;
     static constexpr int OFF_RECV = STAGE_IN_RING ? 0 : OFF_SFX + NUM_STAGES * SF_STAGE;          // 1024-byte aligned
     static constexpr int OFF_BAR = OFF_SFX + NUM_STAGES * SF_STAGE + RECV_BYTES;
-    static constexpr int NUM_BARS = 2 * NUM_STAGES + 7;
+    // Accumulators in tensor memory.  A group-scaled kind rescales every K group's partial product before it is added
+    // (promote_run), so it cycles through a deeper ring of TOK-column buffers; the others keep two whole runs.
+    static constexpr int ACC_BUFS = KIND == KIND_F8G ? (TOK > 64 ? 4 : 8) : 2;
+    static constexpr int ACC_COLS = KIND == KIND_F8G ? TOK : 128;
+    static_assert(ACC_BUFS * ACC_COLS <= TMEM_COLS, "accumulators must fit tensor memory");
+    static constexpr int NUM_BARS = 2 * NUM_STAGES + 2 * ACC_BUFS + 3;
     static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;
     static constexpr int OFF_TABLE = OFF_MISC + 16;                          // first unit of every CTA (+ the end)
-    static constexpr int SMEM_BYTES = OFF_TABLE + (DEC_MAX_CTAS + 2) * 4 + 1024;
+    static constexpr int OFF_TSCALE = (OFF_TABLE + (DEC_MAX_CTAS + 2) * 4 + 15) / 16 * 16;   // [4 warps][2][TOK] token scales
+    static constexpr int SMEM_BYTES = OFF_TSCALE + (KIND == KIND_F8G ? 4 * 2 * TOK * 4 : 0) + 1024;
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared-memory limit");
     static_assert(SMEM_BYTES > 116224, "two CTAs could share an SM and deadlock on tensor-memory allocation");
     static_assert(NUM_STAGES >= 4, "pipeline too shallow");
@@ -92,6 +104,11 @@ __device__ __forceinline__ int dec_unit0(const DecPlan& p, int c) {
 // scratch slot of the run that CTA c starts at unit seg_start: its first run uses slot 2c, a later one 2c+1
 __device__ __forceinline__ int dec_slot(const int* u0, int c, int seg_start) { return seg_start == u0[c] ? 2 * c : 2 * c + 1; }
 
+// Where a CTA starts inside the K stages [kb0, kb0 + len) of a tile (see UnitWalk).
+__device__ __forceinline__ int dec_rotation(int tile, int len) {
+    return static_cast<int>((blockIdx.x * 7u + static_cast<unsigned>(tile) * 3u) % static_cast<unsigned>(len));
+}
+
 // Order in which a CTA visits the (column tile, K stage) units of its run.  Inside each tile the
 // K stages are visited from a CTA-specific starting point, wrapping around: all CTAs need the
 // same activation chunk for the same K stage, and without the offset they would all ask the same
@@ -109,7 +126,7 @@ struct UnitWalk {
             tile = static_cast<int>(u / S);
             kb0 = static_cast<int>(u - static_cast<long long>(tile) * S);
             len = static_cast<int>(min(static_cast<long long>(S - kb0), u_end - u));
-            rot = static_cast<int>((blockIdx.x * 7u + static_cast<unsigned>(tile) * 3u) % static_cast<unsigned>(len));
+            rot = dec_rotation(tile, len);
             i = 0;
         }
         int k = i + rot;
@@ -143,6 +160,97 @@ __device__ __forceinline__ void bulk_send_to_cta(void* dst_local_equiv, const vo
                  : "memory");
 }
 
+// Two accumulators (adjacent tokens) += partial product * scale: fma.rn.f32x2 is two IEEE fused multiply-adds.
+__device__ __forceinline__ void dec_fma2(float& a0, float& a1, float p0, float p1, unsigned long long s2) {
+    unsigned long long a, p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(a0), "f"(a1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(p0), "f"(p1));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(p), "l"(s2));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+}
+
+// Group-scaled FP8: one run (K groups [kb0, kb0 + len) of `tile`, one shared-memory stage each) into registers.
+// This thread's lane of tensor memory is one weight row, i.e. one output column; acc[t] belongs to token t.  Per group
+// acc = p * (sa * sb) + acc for block scales, acc = (p * sa) * sb + acc for per-column ones - the operations of the
+// tiled kernels, in the order the producer visits the groups.  The activation scales of the TOK tokens are fetched
+// DEPTH groups ahead (one token per lane) and handed round through a small per-warp buffer.
+template <int TOK, bool SB_BLOCK, int BUFS>
+__device__ __forceinline__ bool promote_run(const GemmArgs& args, int tile, int kb0, int len, int S, uint32_t tmem_lane,
+                                            uint64_t* acc_full, uint64_t* acc_empty, volatile uint32_t* abort_flag, float* tscale,
+                                            int lane, int nl, uint32_t& step, float (&acc)[TOK]) {
+    constexpr int J = (TOK + 31) / 32;
+    constexpr int DEPTH = TOK > 64 ? 2 : 4;
+    const int rot = dec_rotation(tile, len);
+    const int col = tile * 128 + nl;
+    const float* sb_ptr = SB_BLOCK ? args.gsb + static_cast<size_t>(tile) * S : args.gsb + min(col, args.n - 1);
+    float sa_q[DEPTH][J], sb_q[DEPTH];
+    auto fetch = [&](int i, float (&sa)[J], float& sb) {
+        int kb = i + rot;
+        if (kb >= len) kb -= len;
+        kb += kb0;
+        sb = __ldg(SB_BLOCK ? sb_ptr + kb : sb_ptr + static_cast<size_t>(kb) * args.n);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int t = min(lane + 32 * j, args.m_total - 1);     // rows beyond m_total are computed and never stored
+            sa[j] = __ldg(args.gsa + static_cast<size_t>(t) * S + kb);
+        }
+    };
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) fetch(min(d, len - 1), sa_q[d], sb_q[d]);
+#pragma unroll 1
+    for (int i = 0; i < len; ++i, ++step) {
+        float* ts = tscale + (i & 1) * TOK;
+        const float sb = sb_q[0];
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (TOK >= 32 || lane < TOK) ts[lane + 32 * j] = SB_BLOCK ? __fmul_rn(sa_q[0][j], sb) : sa_q[0][j];
+#pragma unroll
+        for (int d = 0; d + 1 < DEPTH; ++d) {
+            sb_q[d] = sb_q[d + 1];
+#pragma unroll
+            for (int j = 0; j < J; ++j) sa_q[d][j] = sa_q[d + 1][j];
+        }
+        fetch(min(i + DEPTH, len - 1), sa_q[DEPTH - 1], sb_q[DEPTH - 1]);
+        const uint32_t buf = step % BUFS;
+        if (!mbar_wait(acc_full + buf, (step / BUFS) & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+        __syncwarp();
+        tc_fence_after();
+        uint32_t v[2][16];
+        tmem_ld_32x32b_x16(tmem_lane + buf * TOK, v[0]);
+#pragma unroll
+        for (int c = 0; c < TOK / 16; ++c) {
+            tmem_ld_wait();
+            if (c + 1 < TOK / 16) {
+                tmem_ld_32x32b_x16(tmem_lane + buf * TOK + (c + 1) * 16, v[(c + 1) & 1]);
+            } else {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty + buf);
+            }
+            const ulonglong2* s4 = reinterpret_cast<const ulonglong2*>(ts + c * 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const ulonglong2 s = s4[q];
+                float* a = acc + c * 16 + q * 4;
+                const uint32_t* p = v[c & 1] + q * 4;
+                if (SB_BLOCK) {
+                    dec_fma2(a[0], a[1], __uint_as_float(p[0]), __uint_as_float(p[1]), s.x);
+                    dec_fma2(a[2], a[3], __uint_as_float(p[2]), __uint_as_float(p[3]), s.y);
+                } else {
+                    const float4 f = *reinterpret_cast<const float4*>(&s4[q]);
+                    a[0] = fmaf(__fmul_rn(__uint_as_float(p[0]), f.x), sb, a[0]);
+                    a[1] = fmaf(__fmul_rn(__uint_as_float(p[1]), f.y), sb, a[1]);
+                    a[2] = fmaf(__fmul_rn(__uint_as_float(p[2]), f.z), sb, a[2]);
+                    a[3] = fmaf(__fmul_rn(__uint_as_float(p[3]), f.w), sb, a[3]);
+                }
+            }
+        }
+    }
+    return true;
+}
+
 template <int KIND, int TOK>
 __global__ void __launch_bounds__(192, 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -153,8 +261,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
     uint64_t* empty_bar = full_bar + C::NUM_STAGES;
     uint64_t* acc_full = empty_bar + C::NUM_STAGES;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* epi_bar = acc_empty + 2;     // meeting point of the four epilogue warps (bounded, like every wait here)
+    uint64_t* acc_empty = acc_full + C::ACC_BUFS;
+    uint64_t* epi_bar = acc_empty + C::ACC_BUFS;     // meeting point of the four epilogue warps (bounded, like every wait here)
     uint64_t* recv_bar = epi_bar + 1;      // cluster mode, leader: completes when every peer's partial tile has landed
     uint64_t* go_bar = recv_bar + 1;       // cluster mode, peers, ring staging: the leader's ring is free to receive
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
@@ -170,7 +278,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::NUM_STAGES; ++i) { mbar_init(full_bar + i, 1); mbar_init(empty_bar + i, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4); }
+        for (int i = 0; i < C::ACC_BUFS; ++i) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4); }
         mbar_init(epi_bar, 4);
         mbar_init(recv_bar, 1);
         mbar_init(go_bar, 1);
@@ -246,7 +354,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         griddep_wait();
         // instruction descriptor: M = 128 weight rows, N = TOK tokens, both operands K-major
         uint32_t idesc = (static_cast<uint32_t>(TOK >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-        if (KIND == KIND_F8) idesc |= 1u << 4;
+        if (KIND == KIND_F8 || KIND == KIND_F8G) idesc |= 1u << 4;
         if (KIND == KIND_NVF4) idesc |= (1u << 7) | (1u << 10);
         if (KIND == KIND_MXF4) idesc |= (1u << 7) | (1u << 10) | (1u << 23);
         if (KIND == KIND_BF16) idesc |= (1u << 4) | (1u << 7) | (1u << 10);
@@ -254,6 +362,26 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         uint32_t phase = 0;
         bool ok = true;
         int iter = 0;
+        if constexpr (KIND == KIND_F8G) {      // every stage (one K group) is a product of its own
+            uint32_t step = 0;
+            for (long long u = u_begin; u < u_end && ok; ++u, ++step) {
+                const uint32_t buf = step % C::ACC_BUFS;
+                if (!mbar_wait(acc_empty + buf, ((step / C::ACC_BUFS) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
+                if (!mbar_wait(full_bar + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t wdesc = make_desc_sw128(smem_u32(smem + C::OFF_W + stage * C::W_STAGE));
+                const uint64_t xdesc = make_desc_sw128(smem_u32(smem + C::OFF_X + stage * C::X_STAGE));
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mma_f8f6f4(tmem_base + buf * C::ACC_COLS, wdesc + 2 * k, xdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+                    tc_commit(empty_bar + stage);
+                    tc_commit(acc_full + buf);
+                }
+                __syncwarp();
+                if (++stage == C::NUM_STAGES) { stage = 0; phase ^= 1u; }
+            }
+        } else
         for (long long u = u_begin; u < u_end && ok; ++iter) {
             const int tile = static_cast<int>(u / S);
             const int kb0 = static_cast<int>(u - static_cast<long long>(tile) * S);
@@ -324,18 +452,36 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             __syncwarp();
             return met;
         };
+        uint32_t promo_step = 0;
+        auto promote = [&](int tile, int kb0, int len, float (&facc)[TOK]) -> bool {
+            float* tscale = reinterpret_cast<float*>(smem + C::OFF_TSCALE) + (warp - 2) * 2 * TOK;
+            return args.sb_block
+                       ? promote_run<TOK, true, C::ACC_BUFS>(args, tile, kb0, len, S, tmem_base + lane_base, acc_full, acc_empty, abort_flag,
+                                                             tscale, lane, nl, promo_step, facc)
+                       : promote_run<TOK, false, C::ACC_BUFS>(args, tile, kb0, len, S, tmem_base + lane_base, acc_full, acc_empty, abort_flag,
+                                                              tscale, lane, nl, promo_step, facc);
+        };
         if constexpr (C::MAX_PEERS > 0) {
             if (clustered && u_end > u_begin) {
                 // ---- cluster mode: one run inside one tile; the leader (rank 0, lowest K) finishes the tile
                 const int tile = static_cast<int>(u_begin / S);
                 const int col = tile * 128 + nl;
                 const bool col_ok = col < args.n;
-                ok = mbar_wait(acc_full, 0, abort_flag, ST_TIMEOUT_EPILOGUE);
-                tc_fence_after();
+                if constexpr (KIND == KIND_F8G) {
+                    float facc[TOK];
+                    ok = promote(tile, static_cast<int>(u_begin - static_cast<long long>(tile) * S), static_cast<int>(u_end - u_begin), facc);
+                    if (ok) {
+#pragma unroll
+                        for (int t = 0; t < TOK; ++t) recv[t * 128 + nl] = facc[t];
+                    }
+                } else {
+                    ok = mbar_wait(acc_full, 0, abort_flag, ST_TIMEOUT_EPILOGUE);
+                    tc_fence_after();
+                }
                 // Everything below runs once per launch, i.e. from a cold instruction cache, where straight-line
                 // code costs far more than its instruction count suggests (a fully unrolled 64-row finish took
                 // 34 us).  So the accumulator goes to shared memory first and short rolled loops do the rest.
-                if (ok) {
+                if (KIND != KIND_F8G && ok) {
 #pragma unroll 1
                     for (int c = 0; c < TOK / 16; ++c) {
                         uint32_t v[16];
@@ -427,13 +573,25 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const int kb1 = static_cast<int>(min(static_cast<long long>(S), kb0 + (u_end - u)));
             const int acc = iter & 1;
             const uint32_t acc_phase = static_cast<uint32_t>((iter >> 1) & 1);
-            if (!mbar_wait(acc_full + acc, acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
-            tc_fence_after();
+            if constexpr (KIND == KIND_F8G) {      // the run's sums go to this thread's column of the staging tile (rolled loops below)
+                if constexpr (!C::STAGE_IN_RING) {
+                    float facc[TOK];
+                    if (!promote(tile, kb0, kb1 - kb0, facc)) { ok = false; break; }
+#pragma unroll
+                    for (int t = 0; t < TOK; ++t) recv[t * 128 + nl] = facc[t];
+                }
+            } else {
+                if (!mbar_wait(acc_full + acc, acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+                tc_fence_after();
+            }
             const int col = tile * 128 + nl;          // output column = weight row
             const bool col_ok = col < args.n;
             const bool whole = kb0 == 0 && kb1 == S;
             const float cs = (col_ok && args.col_scale != nullptr) ? args.col_scale[col] : 1.0f;
-            if (whole) {
+            if (KIND == KIND_F8G && whole) {
+#pragma unroll 1
+                for (int row = 0; col_ok && row < args.m_total; ++row) store_out(args, row, col, recv[row * 128 + nl], s1, s2, cs);
+            } else if (whole) {
 #pragma unroll 1
                 for (int c = 0; c < TOK / 4; ++c) {      // short body: this code runs from a cold instruction cache
                     uint32_t v[4];
@@ -452,18 +610,23 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             } else {
                 // deliver this run's partial tile, then count in; the last CTA to arrive finishes the tile
                 float* pdst = args.partial + static_cast<size_t>(dec_slot(s_u0, blockIdx.x, static_cast<int>(u))) * (TOK * 128) + nl;
+                if constexpr (KIND == KIND_F8G) {
+#pragma unroll 4
+                    for (int row = 0; row < args.m_total; ++row) __stcg(pdst + row * 128, recv[row * 128 + nl]);
+                } else {
 #pragma unroll 1
-                for (int c = 0; c < TOK / 16; ++c) {
-                    uint32_t v[16];
-                    tmem_ld_32x32b_x16(tmem_base + acc * 128 + c * 16 + lane_base, v);
-                    tmem_ld_wait();
+                    for (int c = 0; c < TOK / 16; ++c) {
+                        uint32_t v[16];
+                        tmem_ld_32x32b_x16(tmem_base + acc * 128 + c * 16 + lane_base, v);
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (c * 16 + i < args.m_total) __stcg(pdst + (c * 16 + i) * 128, __uint_as_float(v[i]));
+                        for (int i = 0; i < 16; ++i)
+                            if (c * 16 + i < args.m_total) __stcg(pdst + (c * 16 + i) * 128, __uint_as_float(v[i]));
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty + acc);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty + acc);
                 const int t0 = tile * S;
                 const int t1 = t0 + S;
                 // the CTAs that hold a piece of this tile: from the one whose run contains unit t0 to the
@@ -683,6 +846,7 @@ size_t decode_scratch_bytes(int kind, const GemmArgs& args, bool* served) {
         case KIND_NVF4: *served = plan_decode_kind<KIND_NVF4>(args, &wanted); break;
         case KIND_MXF4: *served = plan_decode_kind<KIND_MXF4>(args, &wanted); break;
         case KIND_BF16: *served = plan_decode_kind<KIND_BF16>(args, &wanted); break;
+        case KIND_F8G: *served = plan_decode_kind<KIND_F8G>(args, &wanted); break;
         default: break;
     }
     return *served ? wanted : 0;
@@ -705,6 +869,7 @@ int launch_gemm_decode(int kind, const void* A, const void* B, const GemmArgs& a
         case KIND_NVF4: return launch_decode_kind<KIND_NVF4>(A, B, args, st);
         case KIND_MXF4: return launch_decode_kind<KIND_MXF4>(A, B, args, st);
         case KIND_BF16: return launch_decode_kind<KIND_BF16>(A, B, args, st);
+        case KIND_F8G: return launch_decode_kind<KIND_F8G>(A, B, args, st);
         default: return DSL_ERR_ENUM;
     }
 }

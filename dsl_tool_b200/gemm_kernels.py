@@ -119,6 +119,7 @@ def _epilogue(dev, scale_a: Scalar, scale_b: Scalar, out: torch.dtype,
         with torch.cuda.device(dev):
             ws = _lib.workspace(dev, int(_lib.lib().dsl_workspace_bytes(*problem)))
         if ws is not None:
+            keep.append(ws)
             ep.workspace = ws.data_ptr()
             ep.workspace_bytes = ws.numel()
     return ep
@@ -196,7 +197,8 @@ def gemm_fp8_groupwise_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, sa: torc
     nc = _out_cols(n, activation)
     out = torch.empty((M, nc), dtype=_out_dtype(out_dtype), device=dev)
     keep: list = []
-    ep = _epilogue(dev, None, None, out.dtype, row_scale, col_scale, keep, False, activation)
+    ep = _epilogue(dev, None, None, out.dtype, row_scale, col_scale, keep, False, activation,
+                   (_lib.OP_GEMM_FP8_GROUPWISE, M, n, K, groups))
     with torch.cuda.device(dev):
         rc = _lib.lib().dsl_gemm_fp8_groupwise(qa.data_ptr(), qb_nk.data_ptr(), sa.data_ptr(), sb.data_ptr(),
                                                1 if sb_block else 0, out.data_ptr(), nc, M, n, K, _lib.ptr(offs),

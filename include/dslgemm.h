@@ -147,7 +147,7 @@ typedef struct {
  * Bytes of dsl_epilogue.workspace that the GEMM entry point `op` can put to use for a dense M x N x K
  * problem on the CURRENT device (it asks for the device's SM count), header included; 0 when the kernels
  * that serve the problem need no scratch (large M, row groups, decode shapes whose partial tiles are
- * combined inside thread-block clusters, the group-scaled FP8 GEMM).  Decode shapes with more 128-column
+ * combined inside thread-block clusters).  Decode shapes with more 128-column
  * tiles than SMs take 2 partial tiles of TOK x 128 floats per CTA (TOK = 16 or 32 tokens); other
  * problems that would leave more than half of the SMs idle take up to 8 K-slices of M x N floats.
  */

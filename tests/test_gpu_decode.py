@@ -109,3 +109,32 @@ def test_epilogue_scales_and_strided_output(cuda_device):
     got16 = gemm_fp8_quantized(_t(qa), _t(qb), float(sa), float(sb), n=N, row_scale=_t(rs), col_scale=_t(cs),
                                out_dtype="bfloat16")
     assert torch.equal(got16, got.bfloat16())
+
+
+# Group-scaled FP8 (fp32 scales per 128 K) in the streaming kernel: every token bucket with its edges, both weight-scale
+# forms, and every way of cutting the work - clusters of 4 and of 2, one CTA per tile, and past more tiles than SMs runs
+# that cross tile borders - with a ragged last column tile.  Tolerance: an output is a sum of K/128 fp32 terms, each off by
+# at most 2 roundings, added with one rounding each, i.e. (K/128 + 2) * 2^-24 <= 2.7e-6 of the terms' size for K = 5504;
+# the tensor core's sums inside a group keep at least as many bits.  1e-5 leaves a factor of four.
+@pytest.mark.parametrize("sb_block", [True, False])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(2300, 5504), (6400, 1152), (9700, 640), (19100, 640)])
+def test_group_scaled_fp8(cuda_device, sb_block, M, N, K):
+    from dsl_tool_b200 import _lib
+    from dsl_tool_b200.gemm_kernels import gemm_fp8_groupwise_quantized
+    gen = torch.Generator(device="cuda").manual_seed(N + M)
+    def draw(*shape):
+        return torch.randn(shape, generator=gen, device="cuda")
+    qa, qb = (draw(*s).mul_(100).clamp_(-448, 448).to(torch.float8_e4m3fn) for s in ((M, K), (N, K)))
+    sa = draw(M, K // 128).abs_().add_(0.1)
+    sb = draw((N + 127) // 128, K // 128).abs_().add_(0.1) if sb_block else draw(K // 128, N).abs_().add_(0.1)
+    sb_nk = (sb.repeat_interleave(128, 0)[:N] if sb_block else sb.t()).double().repeat_interleave(128, 1)
+    want = (qa.double() * sa.double().repeat_interleave(128, 1)) @ (qb.double() * sb_nk).t()
+    col = draw(N).abs_()
+    args = (qa.view(torch.uint8), qb.view(torch.uint8), sa, sb[None])
+    got = gemm_fp8_groupwise_quantized(*args, n=N, sb_block=sb_block)
+    _lib.check_status()
+    assert float((got - want).norm() / want.norm()) <= 1e-5
+    assert torch.equal(got, gemm_fp8_groupwise_quantized(*args, n=N, sb_block=sb_block))
+    scaled = gemm_fp8_groupwise_quantized(*args, n=N, sb_block=sb_block, out_dtype="bfloat16", row_scale=sa[:, 0], col_scale=col)
+    assert torch.equal(scaled, (got * sa[:, :1] * col).bfloat16())
