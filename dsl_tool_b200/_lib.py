@@ -85,6 +85,7 @@ _SIGNATURES = {
     "dsl_quant_fp8": (_i, [_vp, _i, _ll, _ll, _i, _vp, _i, _vp, _vp, _vp]),
     "dsl_quant_fp4": (_i, [_vp, _i, _ll, _ll, _i, _vp, _i, _vp, _vp, _vp, _i, _vp, _vp]),
     "dsl_quant_fp4_per_token": (_i, [_vp, _i, _ll, _ll, _vp, _vp, _vp, _vp, _i, _vp]),
+    "dsl_pack_kn": (_i, [_vp, _i, _i, _i, _i, _i, _i, _vp, _i, _vp, _vp, ctypes.c_size_t, _vp, _vp]),
     "dsl_transpose_u8": (_i, [_vp, _vp, _i, _i, _vp]),
     "dsl_gemm_fp8": (_i, [_vp, _vp, _vp, _ll, _ll, _i, _i, _vp, _i, ctypes.POINTER(Epilogue), _vp, _vp]),
     "dsl_gemm_fp8_groupwise": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _ll, _ll, _i, _i, _vp, _i,

@@ -88,6 +88,40 @@ int dsl_quant_fp4_per_token(const void* x, int dtype, long long rows, long long 
                                                          groups, as_stream(stream)));
 }
 
+int dsl_pack_kn(const void* w, int dtype, int groups, int K, int N, int format, int interleave, float* scale_io, int scale_given,
+                void* q_out, void* scale_out, size_t scale_bytes, void* ws, void* stream) {
+    if (w == nullptr || q_out == nullptr) return DSL_ERR_NULL;
+    if (dtype < DSL_F32 || dtype > DSL_F16) return DSL_ERR_ENUM;
+    if (groups < 0 || K < 0 || N < 0) return DSL_ERR_SHAPE;
+    int k_multiple;
+    bool has_scale = true, has_tensor_scale = false;
+    size_t need = 0;
+    switch (format) {
+        case DSL_W_NVFP4: k_multiple = 32; has_tensor_scale = true; break;
+        case DSL_W_MXFP4: k_multiple = 32; break;
+        case DSL_W_FP8: k_multiple = 16; has_scale = false; has_tensor_scale = true; break;
+        case DSL_W_FP8_BLOCK128: k_multiple = 16; break;
+        case DSL_W_BF16: k_multiple = 8; has_scale = false; break;
+        default: return DSL_ERR_ENUM;
+    }
+    const int vec = dtype == DSL_F32 ? 4 : 8;
+    if (interleave && N % 2 != 0) return DSL_ERR_SHAPE;
+    const int half = interleave ? N / 2 : 0;
+    if (K % k_multiple != 0 || N % vec != 0 || half % vec != 0) return DSL_ERR_SHAPE;
+    if (groups > 65535 || (N + 127) / 128 > 65535) return DSL_ERR_TOO_LARGE;      // grid dimensions
+    if (!aligned16(w) || !aligned16(q_out) || (has_scale && !aligned16(scale_out))) return DSL_ERR_ALIGN;
+    if (groups == 0 || K == 0 || N == 0) return 0;
+    if (has_scale && scale_out == nullptr) return DSL_ERR_NULL;
+    if (has_tensor_scale && (scale_io == nullptr || (!scale_given && ws == nullptr))) return DSL_ERR_NULL;
+    const size_t tiles = static_cast<size_t>(groups) * ((N + 127) / 128);
+    if (format == DSL_W_NVFP4) need = tiles * ((K / 16 + 3) / 4) * 512;
+    if (format == DSL_W_MXFP4) need = tiles * ((K / 32 + 3) / 4) * 512;
+    if (format == DSL_W_FP8_BLOCK128) need = tiles * ((K + 127) / 128) * sizeof(float);
+    if (scale_bytes < need) return DSL_ERR_TOO_LARGE;
+    return static_cast<int>(launch_pack_kn(w, dtype, groups, K, N, format, half, scale_io, scale_given, static_cast<uint8_t*>(q_out),
+                                           static_cast<uint8_t*>(scale_out), scale_bytes, static_cast<uint32_t*>(ws), as_stream(stream)));
+}
+
 int dsl_transpose_u8(const uint8_t* in, uint8_t* out, int R, int C, void* stream) {
     if (in == nullptr || out == nullptr) return DSL_ERR_NULL;
     if (R < 0 || C < 0) return DSL_ERR_SHAPE;

@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 #include <float.h>
 
+#include "gemm.cuh"
 #include "gemm_tiles.cuh"
 #include "ptx.cuh"
 #include "quant.cuh"
@@ -917,6 +918,237 @@ quant_fp8_tensor_cluster_kernel(const T* __restrict__ x, int nvec, float* __rest
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// ---- weights stored [K, N] (the reference's layout): transposed and quantised in one pass ------
+// One CTA per 128 (output rows) x 128 (K) tile: 16-byte asynchronous copies bring 128 rows of K into shared memory,
+// every thread then reads its chunks of 16 K-consecutive elements down the columns (adjacent lanes hold adjacent
+// columns, so the reads are free of bank conflicts), quantises them exactly as the row-wise kernels above do, and the
+// results leave through a second staging tile so that every row of the output is written in whole 32-byte sectors and
+// every 512-byte scale tile in one piece.  Bound by DRAM: one read of the weight and one write of the result (after an
+// amax pass for the tensor-wide scales), instead of a transposing copy through memory first (read + write of the
+// unquantised weight) and a quantise pass after it.  4096 x 14336 bf16 to NVFP4: 29.3 us, 5.1 TB/s of the 150 MB, where
+// the transposing copy took 272 us and the row-wise quantiser another 30; with the amax pass the call went 294.7 -> 59.8 us.
+// The 128 x 128 tile is one FP8 scale block and whole FP4 scale tiles; 32 KB + 9 KB of shared memory leave five CTAs per SM
+// whose loads and conversions overlap.
+// `half` > 0 folds the gate/up reordering in: output row 2i is source column i, row 2i + 1 is source column half + i.
+enum { PK_NVFP4 = 0, PK_MXFP4 = 1, PK_FP8 = 2, PK_FP8_GIVEN = 3, PK_FP8_BLOCK = 4, PK_BF16 = 5 };
+constexpr int kPackTile = 128;
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// Chunks down one column (fp32) or two adjacent ones (16-bit types) of the staged tile.
+template <typename T> struct ColumnChunks;
+template <> struct ColumnChunks<float> {
+    static constexpr int COLS = 1;
+    static __device__ __forceinline__ void read(const uint32_t* s, Chunk16<float> (&c)[1]) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) c[0].v[i] = __uint_as_float(s[i * kPackTile]);
+    }
+};
+template <> struct ColumnChunks<__nv_bfloat16> {
+    static constexpr int COLS = 2;
+    static __device__ __forceinline__ void read(const uint32_t* s, Chunk16<__nv_bfloat16> (&c)[2]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t a = s[(2 * i) * (kPackTile / 2)], b = s[(2 * i + 1) * (kPackTile / 2)];
+            c[0].w[i] = __byte_perm(a, b, 0x5410);
+            c[1].w[i] = __byte_perm(a, b, 0x7632);
+        }
+    }
+};
+template <> struct ColumnChunks<__half> {
+    static constexpr int COLS = 2;
+    static __device__ __forceinline__ void read(const uint32_t* s, Chunk16<__half> (&c)[2]) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            uint32_t w = s[i * (kPackTile / 2)];
+            const float2 f = __half22float2(*reinterpret_cast<__half2*>(&w));
+            c[0].v[i] = f.x;
+            c[1].v[i] = f.y;
+        }
+    }
+};
+template <typename T>
+__device__ __forceinline__ void chunk_to_bf16(const Chunk16<T>& c, uint4& lo, uint4& hi) {
+    float v[16];
+    c.to_float(v);
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    lo = make_uint4(w[0], w[1], w[2], w[3]);
+    hi = make_uint4(w[4], w[5], w[6], w[7]);
+}
+template <>
+__device__ __forceinline__ void chunk_to_bf16<__nv_bfloat16>(const Chunk16<__nv_bfloat16>& c, uint4& lo, uint4& hi) {
+    lo = make_uint4(c.w[0], c.w[1], c.w[2], c.w[3]);
+    hi = make_uint4(c.w[4], c.w[5], c.w[6], c.w[7]);
+}
+
+template <int FMT> struct PackOut {
+    static constexpr int CHUNK_BYTES = FMT <= PK_MXFP4 ? 8 : (FMT == PK_BF16 ? 32 : 16);     // of 16 elements
+    static constexpr int ROW_BYTES = 8 * CHUNK_BYTES;
+    static constexpr int PITCH = FMT <= PK_MXFP4 ? ROW_BYTES + 8 : ROW_BYTES + 16;
+    static constexpr int SF_BYTES = FMT == PK_NVFP4 ? 1024 : (FMT == PK_MXFP4 ? 512 : 0);    // scale tiles of this CTA
+    static constexpr int BYTES = kPackTile * PITCH + SF_BYTES;
+};
+
+template <typename T, int FMT>
+__global__ void __launch_bounds__(256)
+pack_kn_kernel(const T* __restrict__ w, int K, int N, int half, float* __restrict__ scale_io, const uint32_t* __restrict__ amax_bits,
+               uint8_t* __restrict__ q, uint8_t* __restrict__ scales) {
+    using O = PackOut<FMT>;
+    constexpr int COLS = ColumnChunks<T>::COLS;
+    constexpr int PER_PASS = FMT == PK_MXFP4 ? 2 : 1;          // chunks along K per unit of work: one scale block
+    constexpr int LANE_SETS = kPackTile / COLS / 32;            // passes over the columns
+    constexpr int K_UNITS = 8 / PER_PASS;
+    constexpr int UNITS = LANE_SETS * K_UNITS / 8;              // units of work per warp
+    extern __shared__ __align__(16) uint8_t pack_smem[];
+    __shared__ float red[8];
+    uint32_t* tile = reinterpret_cast<uint32_t*>(pack_smem);                        // [128 K][128 columns]
+    uint8_t* out = pack_smem + kPackTile * kPackTile * sizeof(T);                   // [128 rows][PITCH]
+    uint8_t* sf = out + kPackTile * O::PITCH;
+    const int kt = blockIdx.x, nt = blockIdx.y, g = blockIdx.z;
+    const int k0 = kt * kPackTile, n0 = nt * kPackTile;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        constexpr int VEC = 16 / sizeof(T);
+        constexpr int VECS = kPackTile / VEC;                   // per row of the tile
+        const uint8_t* base = reinterpret_cast<const uint8_t*>(w) + static_cast<size_t>(g) * K * N * sizeof(T);
+#pragma unroll 8
+        for (int i = threadIdx.x; i < kPackTile * VECS; i += 256) {
+            const int r = i / VECS, c = (i % VECS) * VEC;
+            int col;
+            bool ok;
+            if (half > 0) {
+                const int j = (n0 >> 1) + (c & 63);
+                ok = j < half;
+                col = j + (c >= 64 ? half : 0);
+            } else {
+                col = n0 + c;
+                ok = col < N;
+            }
+            ok = ok && k0 + r < K;
+            uint8_t* dst = pack_smem + static_cast<size_t>(i) * 16;
+            if (ok) cp_async16(dst, base + (static_cast<size_t>(k0 + r) * N + col) * sizeof(T));
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    }
+    Nvfp4Scaler scaler;
+    float fs = 0.f;
+    if (FMT == PK_NVFP4) {
+        float gs;
+        if (amax_bits != nullptr) {
+            const float a = __uint_as_float(*amax_bits);
+            gs = a == 0.f ? 1.0f : __fdiv_rn(a, 2688.0f);
+            if (kt == 0 && nt == 0 && g == 0 && threadIdx.x == 0) *scale_io = gs;
+        } else {
+            gs = *scale_io;
+        }
+        scaler.init(gs);
+    }
+    if (FMT == PK_FP8) {
+        fs = fp8_scale_from_amax(__uint_as_float(*amax_bits));
+        if (kt == 0 && nt == 0 && g == 0 && threadIdx.x == 0) *scale_io = fs;
+    }
+    if (FMT == PK_FP8_GIVEN) fs = *scale_io;
+    __syncthreads();
+    Chunk16<T> held[FMT == PK_FP8_BLOCK ? UNITS : 1][COLS];
+    if (FMT == PK_FP8_BLOCK) {      // the block's maximum first; its elements stay in registers
+        float m = 0.f;
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int unit = u * 8 + warp, kc = unit % 8, cset = unit / 8;
+            ColumnChunks<T>::read(tile + (kc * 16 * kPackTile * sizeof(T)) / 4 + cset * 32 + lane, held[FMT == PK_FP8_BLOCK ? u : 0]);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) m = fmaxf(m, held[FMT == PK_FP8_BLOCK ? u : 0][c].amax());
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        if (lane == 0) red[warp] = m;
+        __syncthreads();
+        m = red[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) m = fmaxf(m, red[i]);
+        fs = fp8_scale_from_amax(m);
+        if (threadIdx.x == 0)
+            reinterpret_cast<float*>(scales)[(static_cast<size_t>(g) * gridDim.y + nt) * gridDim.x + kt] = fs;
+    }
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+        const int unit = u * 8 + warp, ku = unit % K_UNITS, cset = unit / K_UNITS;
+        Chunk16<T> ch[PER_PASS][COLS];
+#pragma unroll
+        for (int j = 0; j < PER_PASS; ++j) {
+            if (FMT == PK_FP8_BLOCK) {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) ch[j][c] = held[FMT == PK_FP8_BLOCK ? u : 0][c];
+            } else {
+                ColumnChunks<T>::read(tile + ((ku * PER_PASS + j) * 16 * kPackTile * sizeof(T)) / 4 + cset * 32 + lane, ch[j]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            const int col = (cset * 32 + lane) * COLS + c;                                   // column of the staged tile ...
+            const int row = half > 0 ? ((col & 63) << 1) + (col >> 6) : col;                 // ... and its output row
+            uint8_t* dst = out + row * O::PITCH + ku * PER_PASS * O::CHUNK_BYTES;
+            if (FMT == PK_NVFP4) {
+                float inv;
+                const uint32_t sfb = scaler(ch[0][c].amax(), inv);
+                *reinterpret_cast<uint2*>(dst) = ch[0][c].quant_e2m1(inv);
+                const bool real = n0 + row < N && k0 + ku * 16 < K;                          // padding bytes of a scale tile are zero
+                sf[(ku >> 2) * 512 + (row & 31) * 16 + (row >> 5) * 4 + (ku & 3)] = real ? static_cast<uint8_t>(sfb) : uint8_t(0);
+            } else if (FMT == PK_MXFP4) {
+                const float m = fmaxf(ch[0][c].amax(), ch[PER_PASS - 1][c].amax());
+                int e = static_cast<int>((__float_as_uint(m) >> 23) & 0xFFu) - 129;
+                e = e < -127 ? -127 : e;
+                const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+#pragma unroll
+                for (int j = 0; j < PER_PASS; ++j) *reinterpret_cast<uint2*>(dst + j * 8) = ch[j][c].quant_e2m1(inv);
+                const bool real = n0 + row < N && k0 + ku * 32 < K;
+                sf[(row & 31) * 16 + (row >> 5) * 4 + ku] = real ? static_cast<uint8_t>(e + 127) : uint8_t(0);
+            } else if (FMT == PK_BF16) {
+                uint4 lo, hi;
+                chunk_to_bf16<T>(ch[0][c], lo, hi);
+                reinterpret_cast<uint4*>(dst)[0] = lo;
+                reinterpret_cast<uint4*>(dst)[1] = hi;
+            } else {
+                float v[16];
+                ch[0][c].to_float(v);
+                *reinterpret_cast<uint4*>(dst) = quant16_e4m3<FMT == PK_FP8_GIVEN>(v, fs);
+            }
+        }
+    }
+    __syncthreads();
+    {   // rows of the result, 16 bytes per thread
+        constexpr int VECS = O::ROW_BYTES / 16;
+        const size_t pitch = FMT <= PK_MXFP4 ? static_cast<size_t>(K) / 2 : static_cast<size_t>(K) * (FMT == PK_BF16 ? 2 : 1);
+        const size_t col0 = static_cast<size_t>(kt) * O::ROW_BYTES;
+        uint8_t* qg = q + (static_cast<size_t>(g) * N + n0) * pitch + col0;
+#pragma unroll
+        for (int i = threadIdx.x; i < kPackTile * VECS; i += 256) {
+            const int r = i / VECS, v = i % VECS;
+            if (n0 + r < N && col0 + v * 16 < pitch) {
+                const uint2* s = reinterpret_cast<const uint2*>(out + r * O::PITCH + v * 16);
+                const uint2 a = s[0], b = s[1];
+                *reinterpret_cast<uint4*>(qg + r * pitch + v * 16) = make_uint4(a.x, a.y, b.x, b.y);
+            }
+        }
+    }
+    if (O::SF_BYTES > 0 && threadIdx.x < O::SF_BYTES / 16) {
+        constexpr int ATOMS = O::SF_BYTES / 512;
+        const int katoms = (K / (FMT == PK_NVFP4 ? 16 : 32) + 3) / 4;
+        const int atom = kt * ATOMS + static_cast<int>(threadIdx.x >> 5);
+        if (atom < katoms)
+            reinterpret_cast<uint4*>(scales + ((static_cast<size_t>(g) * gridDim.y + nt) * katoms + atom) * 512)[threadIdx.x & 31] =
+                reinterpret_cast<const uint4*>(sf)[threadIdx.x];
+    }
+}
+
 // ---- byte-matrix transpose ([R, C] -> [C, R]), used to turn a [K, N] weight K-major --------
 __global__ void __launch_bounds__(256) transpose_u8_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out,
                                                            int R, int C) {
@@ -1070,6 +1302,62 @@ cudaError_t launch_quant_nvfp4_per_token(const void* x, int dtype, long long row
         case DSL_F32: return quant_token_typed(static_cast<const float*>(x), rows, cols, gs_out, q, sf, group_offsets, num_groups, st);
         case DSL_BF16: return quant_token_typed(static_cast<const __nv_bfloat16*>(x), rows, cols, gs_out, q, sf, group_offsets, num_groups, st);
         default: return quant_token_typed(static_cast<const __half*>(x), rows, cols, gs_out, q, sf, group_offsets, num_groups, st);
+    }
+}
+
+template <typename T, int FMT>
+static cudaError_t pack_kn_one(const T* w, int groups, int K, int N, int half, float* scale_io, const uint32_t* amax_bits, uint8_t* q,
+                               uint8_t* scales, cudaStream_t st) {
+    constexpr int smem = kPackTile * kPackTile * static_cast<int>(sizeof(T)) + PackOut<FMT>::BYTES;
+    static PerDeviceInt attr_set;   // per device; idempotent
+    const int dev = current_device_slot();
+    if (dev < 0) return cudaErrorInvalidDevice;
+    if (attr_set.v[dev].load(std::memory_order_acquire) == 0) {
+        const cudaError_t e = cudaFuncSetAttribute(pack_kn_kernel<T, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        attr_set.v[dev].store(1, std::memory_order_release);
+    }
+    const dim3 grid((K + kPackTile - 1) / kPackTile, (N + kPackTile - 1) / kPackTile, groups);
+    pack_kn_kernel<T, FMT><<<grid, 256, smem, st>>>(w, K, N, half, scale_io, amax_bits, q, scales);
+    return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t pack_kn_typed(const T* w, int groups, int K, int N, int format, int half, float* scale_io, int scale_given, uint8_t* q,
+                                 uint8_t* scales, size_t scale_bytes, uint32_t* ws, cudaStream_t st) {
+    const uint32_t* amax_bits = nullptr;
+    if ((format == DSL_W_NVFP4 || format == DSL_W_FP8) && !scale_given) {
+        const size_t n = static_cast<size_t>(groups) * K * N;
+        const cudaError_t e = cudaMemsetAsync(ws, 0, 4, st);
+        if (e != cudaSuccess) return e;
+        amax_kernel<T><<<grid_for(n / 16, 256, 148 * 8), 256, 0, st>>>(w, n, ws, (reinterpret_cast<uintptr_t>(w) & 31u) == 0);
+        amax_bits = ws;
+    }
+    if (format == DSL_W_NVFP4 || format == DSL_W_MXFP4) {     // tiles beyond the groups' own (the ragged-group upper bound) read as zero
+        const size_t katoms = (static_cast<size_t>(K) / (format == DSL_W_NVFP4 ? 16 : 32) + 3) / 4;
+        const size_t used = static_cast<size_t>(groups) * ((N + 127) / 128) * katoms * 512;
+        if (scale_bytes > used) {
+            const cudaError_t e = cudaMemsetAsync(scales + used, 0, scale_bytes - used, st);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    switch (format) {
+        case DSL_W_NVFP4: return pack_kn_one<T, PK_NVFP4>(w, groups, K, N, half, scale_io, amax_bits, q, scales, st);
+        case DSL_W_MXFP4: return pack_kn_one<T, PK_MXFP4>(w, groups, K, N, half, nullptr, nullptr, q, scales, st);
+        case DSL_W_FP8:
+            return scale_given ? pack_kn_one<T, PK_FP8_GIVEN>(w, groups, K, N, half, scale_io, nullptr, q, scales, st)
+                               : pack_kn_one<T, PK_FP8>(w, groups, K, N, half, scale_io, amax_bits, q, scales, st);
+        case DSL_W_FP8_BLOCK128: return pack_kn_one<T, PK_FP8_BLOCK>(w, groups, K, N, half, nullptr, nullptr, q, scales, st);
+        default: return pack_kn_one<T, PK_BF16>(w, groups, K, N, half, nullptr, nullptr, q, scales, st);
+    }
+}
+
+cudaError_t launch_pack_kn(const void* w, int dtype, int groups, int K, int N, int format, int half, float* scale_io, int scale_given,
+                           uint8_t* q, uint8_t* scales, size_t scale_bytes, uint32_t* ws, cudaStream_t st) {
+    switch (dtype) {
+        case DSL_F32: return pack_kn_typed(static_cast<const float*>(w), groups, K, N, format, half, scale_io, scale_given, q, scales, scale_bytes, ws, st);
+        case DSL_BF16: return pack_kn_typed(static_cast<const __nv_bfloat16*>(w), groups, K, N, format, half, scale_io, scale_given, q, scales, scale_bytes, ws, st);
+        default: return pack_kn_typed(static_cast<const __half*>(w), groups, K, N, format, half, scale_io, scale_given, q, scales, scale_bytes, ws, st);
     }
 }
 

@@ -14,5 +14,7 @@ cudaError_t launch_quant_fp4(const void* x, int dtype, long long rows, long long
 cudaError_t launch_quant_nvfp4_per_token(const void* x, int dtype, long long rows, long long cols, float* gs_out, uint8_t* q,
                                          uint8_t* sf, size_t sf_bytes, int sf_needs_clear, const int* group_offsets,
                                          int num_groups, cudaStream_t st);
+cudaError_t launch_pack_kn(const void* w, int dtype, int groups, int K, int N, int format, int half, float* scale_io, int scale_given,
+                           uint8_t* q, uint8_t* scales, size_t scale_bytes, uint32_t* ws, cudaStream_t st);
 cudaError_t launch_transpose_u8(const uint8_t* in, uint8_t* out, int R, int C, cudaStream_t st);
 }  // namespace dsl

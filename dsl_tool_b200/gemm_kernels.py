@@ -17,7 +17,7 @@ from typing import Optional, Tuple, Union
 import torch
 
 from . import _lib
-from .quantize import PackedWeight, pack_weight, quantize_fp4, quantize_fp8, transpose_bytes
+from .quantize import PackedWeight, _pack_kn, _pack_kn_serves, pack_weight, quantize_fp4, quantize_fp8, transpose_bytes
 from .weight_store import cached_pack
 
 _FLOAT_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
@@ -503,13 +503,17 @@ def fp8_gemm(A: torch.Tensor, B, scale_a: Scalar = None, scale_b: Scalar = None,
             return gemm_fp8_quantized(qa, w.q, sa, w.scale, n=N, out_dtype=out_dtype, row_scale=row_scale,
                                       col_scale=col_scale, b_static=True)
         return linear(A, w, out_dtype=out_dtype, row_scale=row_scale, col_scale=col_scale)
-    Bnk = B.t().contiguous() if b_layout == "kn" else B.contiguous()
+    w_format = "fp8" if mode == "per_tensor" else "fp8_block128"
+    if b_layout == "kn" and _pack_kn_serves(B.unsqueeze(0), w_format):
+        packed = _pack_kn(B.unsqueeze(0), w_format, scale_b if mode == "per_tensor" else None, False)
+        qb, sb = packed.q, packed.scale
+    else:
+        Bnk = B.t().contiguous() if b_layout == "kn" else B.contiguous()
+        qb, sb = quantize_fp8(Bnk, "per_tensor", scale=scale_b) if mode == "per_tensor" else quantize_fp8(Bnk, "block128")
     if mode == "per_tensor":
         qa, sa = quantize_fp8(A, "per_tensor", scale=scale_a)
-        qb, sb = quantize_fp8(Bnk, "per_tensor", scale=scale_b)
         return gemm_fp8_quantized(qa, qb, sa, sb, n=N, out_dtype=out_dtype, row_scale=row_scale, col_scale=col_scale)
     qa, sa = quantize_fp8(A, "groupwise")
-    qb, sb = quantize_fp8(Bnk, "block128")
     return gemm_fp8_groupwise_quantized(qa, qb, sa, sb, n=N, sb_block=True, out_dtype=out_dtype,
                                         row_scale=row_scale, col_scale=col_scale)
 

@@ -167,6 +167,55 @@ class PackedWeight:
     gate_up_interleaved: bool = False   # rows reordered to (gate_0, up_0, gate_1, up_1, ...) for the fused SwiGLU epilogue
 
 
+_KN_K_MULTIPLE = {"fp8": 16, "fp8_block128": 16, "nvfp4": 32, "mxfp4": 32, "bf16": 8}
+_W_CODES = {"fp8": _lib.W_FP8, "fp8_block128": _lib.W_FP8_BLOCK128, "nvfp4": _lib.W_NVFP4, "mxfp4": _lib.W_MXFP4, "bf16": _lib.W_BF16}
+
+
+def _pack_kn_serves(w: torch.Tensor, format: str, gate_up_interleave: bool = False) -> bool:
+    """Whether the transposing quantiser takes this [G, K, N] weight: its 16-byte loads run along N (every row, and each
+    half of a gate/up pair, a multiple of 16 bytes) and its 16-byte stores along K.  Anything else is transposed first."""
+    G, K, N = w.shape
+    vec = 16 // w.element_size() if w.dtype in (torch.float32, torch.bfloat16, torch.float16) else 0
+    return (vec > 0 and format in _KN_K_MULTIPLE and w.is_contiguous() and w.data_ptr() % 16 == 0 and 0 < G <= 65535
+            and K > 0 and K % _KN_K_MULTIPLE[format] == 0 and 0 < N <= 65535 * 128 and N % (2 * vec if gate_up_interleave else vec) == 0)
+
+
+def _pack_kn(w: torch.Tensor, format: str, global_scale: Union[None, float, torch.Tensor], gate_up_interleave: bool) -> PackedWeight:
+    """w [G, K, N] -> the PackedWeight of its transpose, quantised without a transposed copy in between."""
+    dev = w.device
+    G, K, N = w.shape
+    fp4 = format in ("nvfp4", "mxfp4")
+    q = torch.empty((G * N, K // 2 if fp4 else K), dtype=torch.bfloat16 if format == "bf16" else torch.uint8, device=dev)
+    scale = tensor_scale = None
+    given = 0
+    if format in ("nvfp4", "fp8"):
+        if global_scale is None and format == "nvfp4" and G > 1 and N % 128 != 0:
+            # the ragged-group layout takes its global scale as a given one
+            global_scale = w.abs().amax().float() / 2688.0
+            global_scale = torch.where(global_scale == 0, torch.ones_like(global_scale), global_scale)
+        if global_scale is None:
+            tensor_scale = torch.empty(1, dtype=torch.float32, device=dev)
+        else:
+            tensor_scale = (global_scale.detach().to(device=dev, dtype=torch.float32).reshape(1).clone()
+                            if isinstance(global_scale, torch.Tensor)
+                            else torch.full((1,), float(global_scale), dtype=torch.float32, device=dev))
+            given = 1
+    if fp4:
+        nblk = K // 16 if format == "nvfp4" else K // 32
+        scale = torch.empty(sf_bytes(G * N, nblk, None if G == 1 or N % 128 == 0 else G), dtype=torch.uint8, device=dev)
+    elif format == "fp8_block128":
+        scale = torch.empty((G, (N + 127) // 128, (K + 127) // 128), dtype=torch.float32, device=dev)
+    ws = torch.empty(4, dtype=torch.int32, device=dev) if tensor_scale is not None and not given else None
+    with torch.cuda.device(dev):
+        rc = _lib.lib().dsl_pack_kn(w.data_ptr(), _lib.dtype_code(w.dtype), G, K, N, _W_CODES[format], 1 if gate_up_interleave else 0,
+                                    _lib.ptr(tensor_scale), given, q.data_ptr(), _lib.ptr(scale),
+                                    0 if scale is None else scale.numel() * scale.element_size(), _lib.ptr(ws), _lib.stream_ptr())
+    _lib.check(rc, "dsl_pack_kn")
+    if format == "fp8":
+        return PackedWeight(format, q, tensor_scale, None, G, N, K)
+    return PackedWeight(format, q, scale, tensor_scale, G, N, K)
+
+
 def _pack_weight_impl(w: torch.Tensor, format: str, layout: str = "nk",
                 global_scale: Union[None, float, torch.Tensor] = None, gate_up_interleave: bool = False) -> PackedWeight:
     """Quantise a weight for the GEMM entry points.
@@ -188,6 +237,8 @@ def _pack_weight_impl(w: torch.Tensor, format: str, layout: str = "nk",
     if w.dim() != 3:
         raise ValueError("weight must be 2-D or 3-D")
     if layout == "kn":
+        if _pack_kn_serves(w, format, gate_up_interleave):
+            return _pack_kn(w, format, global_scale, gate_up_interleave)
         w = w.transpose(1, 2)
     if gate_up_interleave:
         if w.shape[1] % 2:

@@ -91,6 +91,23 @@ int dsl_quant_fp4(const void* x, int dtype, long long rows, long long cols, int 
 int dsl_quant_fp4_per_token(const void* x, int dtype, long long rows, long long cols, float* gs_out, uint8_t* q_out,
                             uint8_t* sf_out, const int* group_offsets, int groups, void* stream);
 
+/*
+ * Quantise and lay out a weight stored [G, K, N] (the reference's B[k*N+n], cuda/gemm/fp8_gemm.cu:29-35) as the K-major
+ * [G, N, K] operand of the GEMM entry points: the transpose happens inside the quantiser, so the unquantised weight is
+ * read once (twice when a tensor-wide scale is derived).  Bytes and scales are those of dsl_quant_fp4 / dsl_quant_fp8 on
+ * the transposed weight.
+ *   w          [groups, K, N] of `dtype`, contiguous, 16-byte aligned; rows a multiple of 16 bytes (N % 8, fp32: N % 4)
+ *   format     DSL_W_*; K % 32 == 0 (FP4), K % 16 == 0 (FP8), K % 8 == 0 (BF16: a transposed conversion)
+ *   interleave non-zero: the N columns are [gate; up]; output rows come as gate_0, up_0, gate_1, ... (N even, N/2 as N above)
+ *   scale_io   NVFP4 global scale / per-tensor FP8 scale: 1 float, read when scale_given != 0, else written; other formats NULL
+ *   q_out      [groups, N, K] packed (K/2 bytes FP4, K FP8, 2K BF16 per row)
+ *   scale_out  FP4: scale tiles, ceil(N/128) per group and K tile, in a buffer of scale_bytes (bytes past the tiles are
+ *              zeroed); 128x128 FP8: [groups, ceil(N/128), ceil(K/128)] fp32; else NULL
+ *   ws         4 bytes of device scratch when a tensor-wide scale is derived
+ */
+int dsl_pack_kn(const void* w, int dtype, int groups, int K, int N, int format, int interleave, float* scale_io, int scale_given,
+                void* q_out, void* scale_out, size_t scale_bytes, void* ws, void* stream);
+
 /* Byte-matrix transpose [R, C] -> [C, R]: turns the reference's [K, N] weight layout
  * (cuda/gemm/fp8_gemm.cu:29-35, B[k*N+n]) into the K-major [N, K] the tensor cores read. */
 int dsl_transpose_u8(const uint8_t* in, uint8_t* out, int R, int C, void* stream);
