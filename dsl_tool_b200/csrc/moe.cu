@@ -352,22 +352,32 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ ids, const 
             float acc[VEC];
 #pragma unroll
             for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
-            for (int s = 0; s < k; ++s) {
-                const int r = s_row[s];
-                if (r < 0) continue;
-                const float w = s_w[s];
-                const uint4 v = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(r) * d_model + c0);
-                if (sizeof(TY) == 4) {
-                    const float* f = reinterpret_cast<const float*>(&v);
+            // Eight slots' rows are requested before the first is added (a loop of load, add, load ... keeps one 16-byte
+            // request per thread in flight); the sum still runs in slot order.  16384 tokens x 8 slots x 4096 bf16: 231 us
+            // with an fp32 result and another 54 to round it -> 190 us with bf16 vector stores, 6.3 TB/s of the 1.2 GB.
+            for (int s0 = 0; s0 < k; s0 += 8) {
+                uint4 v[8];
 #pragma unroll
-                    for (int j = 0; j < VEC; ++j) acc[j] = fmaf(w, f[j], acc[j]);
-                } else {
-                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+                for (int j = 0; j < 8; ++j) {
+                    const int r = s0 + j < k ? s_row[s0 + j] : -1;
+                    if (r >= 0) v[j] = __ldcs(reinterpret_cast<const uint4*>(y + static_cast<size_t>(r) * d_model + c0));
+                }
 #pragma unroll
-                    for (int j = 0; j < VEC / 2; ++j) {
-                        const float2 f = __bfloat1622float2(h[j]);
-                        acc[2 * j] = fmaf(w, f.x, acc[2 * j]);
-                        acc[2 * j + 1] = fmaf(w, f.y, acc[2 * j + 1]);
+                for (int j = 0; j < 8; ++j) {
+                    if (s0 + j >= k || s_row[s0 + j] < 0) continue;
+                    const float w = s_w[s0 + j];
+                    if (sizeof(TY) == 4) {
+                        const float* f = reinterpret_cast<const float*>(&v[j]);
+#pragma unroll
+                        for (int i = 0; i < VEC; ++i) acc[i] = fmaf(w, f[i], acc[i]);
+                    } else {
+                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
+#pragma unroll
+                        for (int i = 0; i < VEC / 2; ++i) {
+                            const float2 f = __bfloat1622float2(h[i]);
+                            acc[2 * i] = fmaf(w, f.x, acc[2 * i]);
+                            acc[2 * i + 1] = fmaf(w, f.y, acc[2 * i + 1]);
+                        }
                     }
                 }
             }
@@ -375,6 +385,15 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ ids, const 
                 float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + static_cast<size_t>(t) * d_model + c0);
 #pragma unroll
                 for (int j = 0; j < VEC / 4; ++j) o[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+            } else if (sizeof(TO) == 2 && VEC == 8 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+                uint32_t p[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(acc[(2 * j) % VEC], acc[(2 * j + 1) % VEC]);
+                    p[j] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + static_cast<size_t>(t) * d_model + c0) =
+                    make_uint4(p[0], p[1], p[2], p[3]);
             } else {
 #pragma unroll
                 for (int j = 0; j < VEC; ++j) {

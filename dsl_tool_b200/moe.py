@@ -429,8 +429,8 @@ def moe_forward(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, *,
         red = peer_reducer(x.shape[0], w.down.n, dt, x.device, group)
         moe_partial(x, logits, w, k, renormalize=renormalize, act_global_scale=act_global_scale, out=red.buffer())
         return red.reduce(out_dtype)
-    # shares that travel in bf16 are written in bf16 by the combine itself (fp32 sum, one rounding)
-    direct = partial and exchange_dtype == torch.bfloat16
+    # shares that travel in bf16, and a whole result wanted in bf16, are written so by the combine itself (fp32 sum, one rounding)
+    direct = exchange_dtype == torch.bfloat16 if partial else out_dtype == torch.bfloat16
     out = moe_partial(x, logits, w, k, renormalize=renormalize, out_dtype=torch.bfloat16 if direct else torch.float32,
                       act_global_scale=act_global_scale)
     if partial:

@@ -233,3 +233,26 @@ def test_token_permutation_invariance_at_scale(cuda_device):
     _lib.check_status()
     assert torch.equal(again, base[perm])
     assert torch.isfinite(base).all() and float(base.abs().max()) > 0
+
+
+# The combine's batches of eight slots and its vector stores: slot counts around a batch, both dtypes of rows and result, a
+# row length with and without whole 16-byte vectors, and an expert range that leaves slots out.  The sum runs in slot order
+# with one fused multiply-add per slot, so fp32 arithmetic in that order gives it to the bit up to the fma's single rounding:
+# k roundings of 2^-24 relative to the terms' size on either side.
+@pytest.mark.parametrize("k", [1, 8, 9, 17])
+@pytest.mark.parametrize("Dm", [264, 20])
+@pytest.mark.parametrize("y_dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_combine_slot_batches(cuda_device, k, Dm, y_dtype, out_dtype):
+    gen = torch.Generator(device="cuda").manual_seed(k * Dm)
+    T, E, first, last = 37, 24, 3, 20
+    ids = torch.rand((T, E), generator=gen, device="cuda").argsort(1)[:, :k].int().contiguous()
+    w = torch.rand((T, k), generator=gen, device="cuda")
+    p = moe.plan(ids, w, E)
+    y = torch.randn((T * k, Dm), generator=gen, device="cuda").to(y_dtype)
+    got = moe.combine(p, y, first, last, out_dtype=out_dtype)
+    rows = (p.dest.view(T, k).long() - int(p.offsets[first])).clamp_(0, T * k - 1)
+    local = ((ids >= first) & (ids < last)).double()
+    terms = (w.double() * local)[:, :, None] * y.double()[rows]
+    want = terms.sum(1)
+    bound = (k + 1) * 2.0 ** -24 * terms.abs().sum(1) + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((got.double() - want).abs() <= bound + 1e-30).all())
