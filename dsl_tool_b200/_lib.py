@@ -56,6 +56,7 @@ class Epilogue(ctypes.Structure):
         ("out_gs_host", ctypes.c_float),
         ("out_gs_dev", ctypes.c_void_p),
         ("act_scale_per_token", ctypes.c_int),
+        ("b_is_kn", ctypes.c_int),
     ]
 
 
@@ -94,6 +95,7 @@ _SIGNATURES = {
                           ctypes.POINTER(Epilogue), _vp, _vp]),
     "dsl_gemm_fp4_static_scratch": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _ll, _ll, _i, _i,
                                          ctypes.POINTER(Epilogue), _vp, _vp]),
+    "dsl_gemm_kn_served": (_i, [_i, _ll, _i, _i, _i]),
     "dsl_workspace_bytes": (ctypes.c_size_t, [_i, _ll, _i, _i, _i]),
     "dsl_linear_scratch_bytes": (ctypes.c_size_t, [_i, _ll, _i, _i]),
     "dsl_linear": (_i, [_vp, _i, _ll, ctypes.POINTER(Weight), _vp, _vp, ctypes.c_size_t, _vp, _ll,

@@ -166,6 +166,7 @@ static int fill_common(GemmArgs& a, const void* A, const void* B, void* C, long 
     a.status = status;
     a.b_static = ep->b_is_static != 0;
     a.act = ep->activation;
+    a.b_kn = ep->b_is_kn != 0;
     if (ep->out_dtype == DSL_OUT_NVFP4) {
         a.out_sf = static_cast<uint8_t*>(ep->out_sf);
         a.out_gs = ep->out_gs_host;
@@ -187,6 +188,7 @@ int dsl_gemm_fp8(const uint8_t* A, const uint8_t* B, void* C, long long ldc, lon
     int rc = fill_common(a, A, B, C, ldc, M_total, N, K, group_offsets, groups, ep, status);
     if (rc != 0) return rc;
     a.scale_product = 0;   // (acc * scale_a) * scale_b, as the registered reference kernel does
+    if (a.b_kn && M_total > 0 && N > 0 && !kn_served(KIND_F8, a)) return DSL_ERR_SHAPE;
     return launch_gemm(KIND_F8, A, B, a, as_stream(stream));
 }
 
@@ -197,6 +199,7 @@ int dsl_gemm_bf16(const void* A, const void* B, void* C, long long ldc, long lon
     int rc = fill_common(a, A, B, C, ldc, M_total, N, 2ll * K, group_offsets, groups, ep, status);
     if (rc != 0) return rc;
     a.scale_product = 0;
+    if (a.b_kn && M_total > 0 && N > 0 && !kn_served(KIND_BF16, a)) return DSL_ERR_SHAPE;
     return launch_gemm(KIND_BF16, A, B, a, as_stream(stream));
 }
 
@@ -213,6 +216,7 @@ int dsl_gemm_fp8_groupwise(const uint8_t* A, const uint8_t* B, const float* sa, 
     a.gsb = sb;
     a.sb_block = sb_block != 0;
     a.scale_product = 0;
+    if (a.b_kn && M_total > 0 && N > 0 && !kn_served(KIND_F8G, a)) return DSL_ERR_SHAPE;
     return launch_gemm_fp8_groupwise(A, B, a, as_stream(stream));
 }
 
@@ -226,6 +230,7 @@ int dsl_gemm_fp4(const uint8_t* A, const uint8_t* B, const uint8_t* sfa, const u
     if (!aligned16(sfa) || !aligned16(sfb)) return DSL_ERR_ALIGN;
     int rc = fill_common(a, A, B, C, ldc, M_total, N, K / 2, group_offsets, groups, ep, status);
     if (rc != 0) return rc;
+    if (a.b_kn) return DSL_ERR_ENUM;         // packed pairs run along K
     const int nblk = format == DSL_FP4_NV ? K / 16 : K / 32;
     a.sfa = sfa;
     a.sfb = sfb;
@@ -235,28 +240,42 @@ int dsl_gemm_fp4(const uint8_t* A, const uint8_t* B, const uint8_t* sfa, const u
     return launch_gemm(format == DSL_FP4_NV ? KIND_NVF4 : KIND_MXF4, A, B, a, as_stream(stream));
 }
 
-size_t dsl_workspace_bytes(int op, long long M, int N, int K, int groups) {
-    if (M <= 0 || N <= 0 || K <= 0 || M > 0x7FFFFFFFll) return 0;
-    if (groups > 1) return 0;                         // row groups: no kernel uses scratch
+// The problem as launch_gemm would see it with all the workspace it could want; false for an op that takes none.
+static bool problem_of(int op, long long M, int N, int K, int* kind, GemmArgs* a) {
+    if (M <= 0 || N <= 0 || K <= 0 || M > 0x7FFFFFFFll) return false;
     long long k_bytes;
-    int kind;
     switch (op) {
-        case DSL_OP_GEMM_FP8: kind = KIND_F8; k_bytes = K; break;
-        case DSL_OP_GEMM_BF16: kind = KIND_BF16; k_bytes = 2ll * K; break;
-        case DSL_OP_GEMM_FP4_NV: kind = KIND_NVF4; k_bytes = K / 2; break;
-        case DSL_OP_GEMM_FP4_MX: kind = KIND_MXF4; k_bytes = K / 2; break;
-        case DSL_OP_GEMM_FP8_GROUPWISE: kind = KIND_F8G; k_bytes = K; break;
-        default: return 0;                            // the quantisers use none
+        case DSL_OP_GEMM_FP8: *kind = KIND_F8; k_bytes = K; break;
+        case DSL_OP_GEMM_BF16: *kind = KIND_BF16; k_bytes = 2ll * K; break;
+        case DSL_OP_GEMM_FP4_NV: *kind = KIND_NVF4; k_bytes = K / 2; break;
+        case DSL_OP_GEMM_FP4_MX: *kind = KIND_MXF4; k_bytes = K / 2; break;
+        case DSL_OP_GEMM_FP8_GROUPWISE: *kind = KIND_F8G; k_bytes = K; break;
+        default: return false;                        // the quantisers use none
     }
-    if (k_bytes <= 0 || k_bytes > 0x7FFFFFFFll) return 0;
-    GemmArgs a{};
-    a.m_total = static_cast<int>(M);
-    a.n = N;
-    a.k_bytes = static_cast<int>(k_bytes);
-    a.num_groups = 1;
-    a.partial = reinterpret_cast<float*>(uintptr_t(16));   // "a workspace is there": never dereferenced
-    a.partial_bytes = ~size_t(0) >> 2;
+    if (k_bytes <= 0 || k_bytes > 0x7FFFFFFFll) return false;
+    *a = GemmArgs{};
+    a->m_total = static_cast<int>(M);
+    a->n = N;
+    a->k_bytes = static_cast<int>(k_bytes);
+    a->num_groups = 1;
+    a->partial = reinterpret_cast<float*>(uintptr_t(16));   // "a workspace is there": never dereferenced
+    a->partial_bytes = ~size_t(0) >> 2;
+    return true;
+}
+
+size_t dsl_workspace_bytes(int op, long long M, int N, int K, int groups) {
+    GemmArgs a;
+    int kind;
+    if (groups > 1 || !problem_of(op, M, N, K, &kind, &a)) return 0;      // row groups: no kernel uses scratch
     return gemm_workspace_bytes(kind, a);
+}
+
+int dsl_gemm_kn_served(int op, long long M, int N, int K, int groups) {
+    GemmArgs a;
+    int kind;
+    if (!problem_of(op, M, N, K, &kind, &a)) return 0;
+    if (groups > 1) a.group_offsets = reinterpret_cast<const int*>(uintptr_t(16));   // "row groups": never dereferenced
+    return kn_served(kind, a) ? 1 : 0;
 }
 
 int dsl_selftest_bounded_wait(uint32_t* status, unsigned limit_us, void* stream) {

@@ -422,6 +422,10 @@ bool make_tmap_u8(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, ui
     return true;
 }
 
+bool make_tmap_kn(CUtensorMap* m, const void* base, int n, long long k, int groups, int elem, uint32_t box_k) {
+    return make_tmap_u8(m, base, static_cast<uint64_t>(n) * elem, static_cast<uint64_t>(k), groups, 128, box_k);
+}
+
 int sm_count() {
     static PerDeviceInt cache;   // 0 = not asked yet
     const int dev = current_device_slot();
@@ -520,6 +524,19 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args) {
     const int split_k = choose_split_k(args, max_tiles);
     if (split_k <= 1) return 0;
     return DSL_WS_HEADER_BYTES + static_cast<size_t>(split_k) * args.m_total * args.n * sizeof(float);
+}
+
+// FP8 and BF16 tiles of a [K, N] operand arrive as 128 bytes of N x one stage of K and go to the tensor core as they are
+// (MN-major); the row pitch of the tensor map wants N in whole 16-byte vectors.  FP4 pairs run along K, so those cannot.
+// Against transposing B first, same bits: 1024^3 FP8 bytes 44.4 -> 30.2 us a call (GEMM alone 13.8 -> 12.4 us), grouped
+// bf16 8 x 384 x 2048 x 1408 66.5 -> 48.2 us (the transpose was 16.6 us; the GEMM takes 29 us either way).
+bool kn_served(int kind, const GemmArgs& args) {
+    if (kind != KIND_F8 && kind != KIND_BF16 && kind != KIND_F8G) return false;
+    const int elem = kind == KIND_BF16 ? 2 : 1;
+    if (args.n <= 0 || args.m_total <= 0 || (static_cast<long long>(args.n) * elem) % 16 != 0 || forced_kernel() != 0) return false;
+    bool decode = false;
+    decode_scratch_bytes(kind, args, &decode);
+    return decode || (args.m_total > 128 && args.n >= 256);
 }
 
 int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st) {

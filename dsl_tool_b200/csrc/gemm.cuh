@@ -41,6 +41,7 @@ struct GemmArgs {
                                  // after its first DSL_WS_HEADER_BYTES
     size_t partial_bytes;        // capacity of `partial`
     unsigned long long* ws_words;   // the workspace's header: DSL_WS_HEADER_BYTES / 8 arrival words (gemm_decode.cu)
+    int b_kn;                    // 1: B is given [G, K, N] (N contiguous) and read MN-major (16- and 8-bit kinds, see kn_served)
     int b_static;                // B was complete before the preceding kernel of the stream was launched
     int act;                     // DSL_ACT_*: SWIGLU turns column pairs (gate, up) into one output column
     uint8_t* out_sf;             // non-null: the result is quantised to NVFP4 (c = packed bytes, out_sf = scale tiles)
@@ -78,6 +79,9 @@ int launch_gemm_decode(int kind, const void* A, const void* B, const GemmArgs& a
 // combines inside clusters or does not serve the problem (*served says which).
 size_t decode_scratch_bytes(int kind, const GemmArgs& args, bool* served);
 size_t gemm_workspace_bytes(int kind, const GemmArgs& args);
+// Whether a problem whose B is stored [K, N] can be multiplied without transposing B first (the CTA-pair kernels and the
+// weight-streaming kernel read it MN-major; the 1-CTA kernels do not).
+bool kn_served(int kind, const GemmArgs& args);
 int choose_split_k(const GemmArgs& args, long long tiles);
 int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st);
 int launch_gemm_pair(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st);
@@ -86,6 +90,8 @@ int groupwise_pair_schedule_host(const int* group_offsets, int groups, int m_tot
                                  int* out, int max_items);
 int launch_gemm_fp8_groupwise(const void* A, const void* B, GemmArgs args, cudaStream_t st);
 int launch_bounded_wait_selftest(uint32_t* status, unsigned limit_us, cudaStream_t st);
+// [groups][K][N] elements of `elem` bytes: boxes of 128 bytes of N x box_k rows of K (the MN-major operand tile)
+bool make_tmap_kn(CUtensorMap* m, const void* base, int n, long long k, int groups, int elem, uint32_t box_k);
 bool make_tmap_u8(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box0,
                   uint32_t box1);
 

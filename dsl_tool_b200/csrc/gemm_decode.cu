@@ -321,7 +321,15 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 int atoms = 0;
                 if (C::SF_ATOMS > 0) atoms = min(C::SF_ATOMS, args.sf_katoms - kb * C::SF_ATOMS);
                 mbar_arrive_expect_tx(full_bar + st, C::W_STAGE + C::X_STAGE + 2 * atoms * 512);
-                tma_load_2d(smem + C::OFF_W + st * C::W_STAGE, &tmap_w, full_bar + st, kb * STAGE_KB, tile * 128);
+                if (C::SF_ATOMS == 0 && args.b_kn) {    // blocks of 128 bytes of N x one stage of K, side by side
+                    constexpr int ELEM = KIND == KIND_BF16 ? 2 : 1;
+#pragma unroll
+                    for (int j = 0; j < ELEM; ++j)
+                        tma_load_3d(smem + C::OFF_W + st * C::W_STAGE + j * (C::W_STAGE / ELEM), &tmap_w, full_bar + st,
+                                    tile * 128 * ELEM + j * 128, kb * (STAGE_KB / ELEM), 0);
+                } else {
+                    tma_load_2d(smem + C::OFF_W + st * C::W_STAGE, &tmap_w, full_bar + st, kb * STAGE_KB, tile * 128);
+                }
                 if (C::SF_ATOMS > 0)
                     bulk_load(smem + C::OFF_SFW + st * C::SF_STAGE,
                               args.sfb + (static_cast<size_t>(tile) * args.sf_katoms + static_cast<size_t>(kb) * C::SF_ATOMS) * 512,
@@ -358,6 +366,11 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (KIND == KIND_NVF4) idesc |= (1u << 7) | (1u << 10);
         if (KIND == KIND_MXF4) idesc |= (1u << 7) | (1u << 10) | (1u << 23);
         if (KIND == KIND_BF16) idesc |= (1u << 4) | (1u << 7) | (1u << 10);
+        // weight given [K, N]: the M side is MN-major (bit 15), 32 bytes of K are 16 / 32 rows of 128 bytes
+        const bool w_kn = C::SF_ATOMS == 0 && args.b_kn != 0;
+        if (w_kn) idesc |= 1u << 15;
+        const uint64_t w_step = w_kn ? (KIND == KIND_BF16 ? 16 * 128 : 32 * 128) >> 4 : 2;
+        const uint32_t w_block = w_kn && KIND == KIND_BF16 ? C::W_STAGE / 2 : 0;
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -369,12 +382,12 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 if (!mbar_wait(acc_empty + buf, ((step / C::ACC_BUFS) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                 if (!mbar_wait(full_bar + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t wdesc = make_desc_sw128(smem_u32(smem + C::OFF_W + stage * C::W_STAGE));
+                const uint64_t wdesc = make_desc_mn_sw128(smem_u32(smem + C::OFF_W + stage * C::W_STAGE), w_block);
                 const uint64_t xdesc = make_desc_sw128(smem_u32(smem + C::OFF_X + stage * C::X_STAGE));
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        mma_f8f6f4(tmem_base + buf * C::ACC_COLS, wdesc + 2 * k, xdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+                        mma_f8f6f4(tmem_base + buf * C::ACC_COLS, wdesc + w_step * k, xdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
                     tc_commit(empty_bar + stage);
                     tc_commit(acc_full + buf);
                 }
@@ -406,15 +419,15 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                             tc_cp_32x128b_warpx4(tmem_base + DEC_SFX_COL + i * 4, make_desc_sf(sfx_addr + i * 512));
                         }
                     }
-                    const uint64_t wdesc = make_desc_sw128(w_addr);
+                    const uint64_t wdesc = make_desc_mn_sw128(w_addr, w_block);
                     const uint64_t xdesc = make_desc_sw128(x_addr);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {   // 4 x 32 bytes of K per stage
                         const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
                         if (KIND == KIND_F8) {
-                            mma_f8f6f4(d_tmem, wdesc + 2 * k, xdesc + 2 * k, idesc, accum);
+                            mma_f8f6f4(d_tmem, wdesc + w_step * k, xdesc + 2 * k, idesc, accum);
                         } else if (KIND == KIND_BF16) {
-                            mma_f16(d_tmem, wdesc + 2 * k, xdesc + 2 * k, idesc, accum);
+                            mma_f16(d_tmem, wdesc + w_step * k, xdesc + 2 * k, idesc, accum);
                         } else if (KIND == KIND_NVF4) {
                             mma_nvf4(d_tmem, wdesc + 2 * k, xdesc + 2 * k, idesc, tmem_base + DEC_SFW_COL + k * 4,
                                      tmem_base + DEC_SFX_COL + k * 4, accum);
@@ -789,7 +802,12 @@ static int launch_decode_one(const void* A, const void* B, const GemmArgs& args,
     if (!plan_decode<KIND, TOK>(args, plan, &wanted)) return DSL_NOT_SERVED;
     plan.epoch = next_epoch();
     CUtensorMap tw, tx;
-    if (!make_tmap_u8(&tw, B, args.k_bytes, args.n, 0, STAGE_KB, 128)) return DSL_ERR_DRIVER;
+    if (args.b_kn) {
+        constexpr int ELEM = KIND == KIND_BF16 ? 2 : 1;
+        if (!make_tmap_kn(&tw, B, args.n, args.k_bytes / ELEM, 1, ELEM, STAGE_KB / ELEM)) return DSL_ERR_DRIVER;
+    } else if (!make_tmap_u8(&tw, B, args.k_bytes, args.n, 0, STAGE_KB, 128)) {
+        return DSL_ERR_DRIVER;
+    }
     if (!make_tmap_u8(&tx, A, args.k_bytes, args.m_total, 0, STAGE_KB, TOK)) return DSL_ERR_DRIVER;
     static PerDeviceInt attr_set;   // per device; idempotent, a race here only repeats the same call
     const int dev = current_device_slot();

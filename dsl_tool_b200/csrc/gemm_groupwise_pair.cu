@@ -300,6 +300,9 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
                     if (narrow)
                         tma_load_3d(smem + OFF_B + stage * B_STAGE, &tmap_b_narrow, full_bar + stage, kb * STAGE_KB,
                                     ti.n0 + (NARROW_N / 2) * static_cast<int>(rank), ti.group);
+                    else if (args.b_kn)     // 128 columns x 128 rows of K (whole tiles only)
+                        tma_load_3d(smem + OFF_B + stage * B_STAGE, &tmap_b, full_bar + stage, ti.n0 + 128 * static_cast<int>(rank),
+                                    kb * STAGE_KB, ti.group);
                     else
                         tma_load_3d(smem + OFF_B + stage * B_STAGE, &tmap_b, full_bar + stage, kb * STAGE_KB,
                                     ti.n0 + 128 * static_cast<int>(rank), ti.group);
@@ -310,7 +313,9 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
         }
     } else if (warp == 1) {
         if (rank == 0) {
-            const uint32_t idesc_full = (1u << 4) | (static_cast<uint32_t>(TILE_N >> 3) << 17) |
+            // B MN-major: bit 16 of the instruction descriptor, 32 elements of K are 32 rows of 128 bytes
+            const uint64_t b_step = args.b_kn ? 32 * 128 >> 4 : 2;
+            const uint32_t idesc_full = (1u << 4) | (args.b_kn ? 1u << 16 : 0u) | (static_cast<uint32_t>(TILE_N >> 3) << 17) |
                                         (static_cast<uint32_t>(TILE_M >> 4) << 24);   // E4M3 x E4M3 -> fp32
             const uint32_t idesc_narrow = (1u << 4) | (static_cast<uint32_t>(NARROW_N >> 3) << 17) |
                                           (static_cast<uint32_t>(TILE_M >> 4) << 24);
@@ -347,7 +352,7 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            mma_f8f6f4_pair(tmem_base + p * buf_cols, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+                            mma_f8f6f4_pair(tmem_base + p * buf_cols, adesc + 2 * k, bdesc + b_step * k, idesc, k > 0 ? 1u : 0u);
                         tc_commit_pair(empty_bar + stage);
                         tc_commit_pair(acc_full + p);
                     }
@@ -411,8 +416,13 @@ static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cu
     CUtensorMap ta, tb, tbn;
     const int groups = args.group_offsets != nullptr ? args.num_groups : 1;
     if (!make_tmap_u8(&ta, A, args.k_bytes, args.m_total, 0, STAGE_KB, 128)) return DSL_ERR_DRIVER;
-    if (!make_tmap_u8(&tb, B, args.k_bytes, args.n, groups, STAGE_KB, 128)) return DSL_ERR_DRIVER;
-    if (!make_tmap_u8(&tbn, B, args.k_bytes, args.n, groups, STAGE_KB, gwp::NARROW_N / 2)) return DSL_ERR_DRIVER;
+    if (args.b_kn) {
+        if (!make_tmap_kn(&tb, B, args.n, args.k_bytes, groups, 1, STAGE_KB)) return DSL_ERR_DRIVER;
+        tbn = tb;       // never used: whole tiles only
+    } else {
+        if (!make_tmap_u8(&tb, B, args.k_bytes, args.n, groups, STAGE_KB, 128)) return DSL_ERR_DRIVER;
+        if (!make_tmap_u8(&tbn, B, args.k_bytes, args.n, groups, STAGE_KB, gwp::NARROW_N / 2)) return DSL_ERR_DRIVER;
+    }
     static PerDeviceInt clusters_of;   // per kernel instantiation and device; idempotent set-up
     const int dev = current_device_slot();
     if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
@@ -499,7 +509,7 @@ int launch_gemm_fp8_groupwise_pair(const void* A, const void* B, GemmArgs args, 
     if (args.band <= 0) args.band = 8;
     {   // DSLGEMM_WHOLE_TILES=1 keeps every tile whole (for measurements)
         static const int whole = [] { const char* e = getenv("DSLGEMM_WHOLE_TILES"); return (e != nullptr && e[0] == '1') ? 1 : 0; }();
-        args.whole_tiles_only = whole;
+        args.whole_tiles_only = whole || args.b_kn;      // a 32-column half of a piece is no whole 128-byte block of an MN-major tile
     }
     // two instantiations: the plain epilogue keeps the promotion loop free of spills, the activation one is larger
     if (args.act != DSL_ACT_NONE)

@@ -206,8 +206,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     mbar_arrive_expect_tx(full_bar + stage, bytes);
                     tma_load_2d(smem + C::OFF_A + stage * C::A_STAGE, &tmap_a, full_bar + stage, kb * STAGE_KB,
                                 ti.row0 + 128 * static_cast<int>(rank));
-                    tma_load_3d(smem + C::OFF_B + stage * C::B_STAGE, &tmap_b, full_bar + stage, kb * STAGE_KB,
-                                ti.n0 + 128 * static_cast<int>(rank), ti.group);
+                    if (C::SF_ATOMS == 0 && args.b_kn) {    // blocks of 128 bytes of N x one stage of K, side by side
+                        constexpr int ELEM = KIND == KIND_BF16 ? 2 : 1;
+#pragma unroll
+                        for (int j = 0; j < ELEM; ++j)
+                            tma_load_3d(smem + C::OFF_B + stage * C::B_STAGE + j * (C::B_STAGE / ELEM), &tmap_b, full_bar + stage,
+                                        (ti.n0 + 128 * static_cast<int>(rank)) * ELEM + j * 128, kb * (STAGE_KB / ELEM), ti.group);
+                    } else {
+                        tma_load_3d(smem + C::OFF_B + stage * C::B_STAGE, &tmap_b, full_bar + stage, kb * STAGE_KB,
+                                    ti.n0 + 128 * static_cast<int>(rank), ti.group);
+                    }
                     if (C::SF_ATOMS > 0) {
                         const size_t katom0 = static_cast<size_t>(kb) * C::SF_ATOMS;
                         if (sfa_valid)
@@ -234,6 +242,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (KIND == KIND_NVF4) idesc |= (1u << 7) | (1u << 10);
             if (KIND == KIND_MXF4) idesc |= (1u << 7) | (1u << 10) | (1u << 23);
             if (KIND == KIND_BF16) idesc |= (1u << 4) | (1u << 7) | (1u << 10);
+            // B MN-major: bit 16 of the instruction descriptor, 32 bytes of K are 16 / 32 rows of 128 bytes
+            const bool b_kn = C::SF_ATOMS == 0 && args.b_kn != 0;
+            if (b_kn) idesc |= 1u << 16;
+            const uint64_t b_step = b_kn ? (KIND == KIND_BF16 ? 16 * 128 : 32 * 128) >> 4 : 2;
+            const uint32_t b_block = b_kn && KIND == KIND_BF16 ? C::B_STAGE / 2 : 0;
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -255,7 +268,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     const uint32_t sfa_addr = smem_u32(smem + C::OFF_SFA + stage * C::SFA_STAGE);
                     const uint32_t sfb_addr = smem_u32(smem + C::OFF_SFB + stage * C::SFB_STAGE);
                     const uint64_t adesc = make_desc_sw128(a_addr);
-                    const uint64_t bdesc = make_desc_sw128(b_addr);
+                    const uint64_t bdesc = make_desc_mn_sw128(b_addr, b_block);
                     if (elect_one()) {
                         if (C::SF_ATOMS > 0) {
 #pragma unroll
@@ -271,9 +284,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                         for (int k = 0; k < 4; ++k) {
                             const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
                             if (KIND == KIND_F8) {
-                                mma_f8f6f4_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+                                mma_f8f6f4_pair(d_tmem, adesc + 2 * k, bdesc + b_step * k, idesc, accum);
                             } else if (KIND == KIND_BF16) {
-                                mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+                                mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + b_step * k, idesc, accum);
                             } else if (KIND == KIND_NVF4) {
                                 mma_nvf4_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, tmem_base + pr::SFA_COL + k * 4,
                                               tmem_base + pr::SFB_COL + k * 8, accum);
@@ -388,7 +401,12 @@ static int launch_pair_one(const void* A, const void* B, const GemmArgs& args, l
     CUtensorMap ta, tb;
     const int groups = args.group_offsets != nullptr ? args.num_groups : 1;
     if (!make_tmap_u8(&ta, A, args.k_bytes, args.m_total, 0, STAGE_KB, 128)) return DSL_ERR_DRIVER;
-    if (!make_tmap_u8(&tb, B, args.k_bytes, args.n, groups, STAGE_KB, 128)) return DSL_ERR_DRIVER;
+    if (args.b_kn) {
+        constexpr int ELEM = KIND == KIND_BF16 ? 2 : 1;
+        if (!make_tmap_kn(&tb, B, args.n, args.k_bytes / ELEM, groups, ELEM, STAGE_KB / ELEM)) return DSL_ERR_DRIVER;
+    } else if (!make_tmap_u8(&tb, B, args.k_bytes, args.n, groups, STAGE_KB, 128)) {
+        return DSL_ERR_DRIVER;
+    }
     static PerDeviceInt clusters_of;   // per kernel instantiation and device; idempotent set-up
     const int dev = current_device_slot();
     if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);

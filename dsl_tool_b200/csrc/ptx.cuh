@@ -322,6 +322,12 @@ __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t smem_addr) {
     d |= 2ull << 61;
     return d;
 }
+// The same for an MN-major operand tile: rows of 128 bytes of the M / N dimension, one row per K element, 128-byte
+// swizzle (what a TMA box of 128 bytes of N x K rows produces).  Eight K rows are 1024 bytes; `block_bytes` separates the
+// tile's 128-byte wide column blocks (bits [16,30): 64 elements of a 16-bit type; unused when one block covers the tile).
+__device__ __forceinline__ uint64_t make_desc_mn_sw128(uint32_t smem_addr, uint32_t block_bytes) {
+    return make_desc_sw128(smem_addr) | (static_cast<uint64_t>((block_bytes >> 4) & 0x3FFFu) << 16);
+}
 // Descriptor for a 512-byte scale-factor tile (32 rows x 16 bytes, no swizzle): 8-row core
 // matrices are 128 bytes apart.
 __device__ __forceinline__ uint64_t make_desc_sf(uint32_t smem_addr) {

@@ -142,6 +142,14 @@ def _offsets_arg(offsets: Optional[torch.Tensor], dev) -> Tuple[Optional[torch.T
     return offsets, groups
 
 
+def _kn_direct(op: int, b: torch.Tensor, M: int, groups: int = 1) -> bool:
+    """Whether the tensor cores read this [K, N] / [G, K, N] operand where it lies (rows in whole 16-byte vectors, a problem
+    of the kernels that do); everything else is transposed first."""
+    K, N = b.shape[-2:]
+    return (b.is_contiguous() and b.data_ptr() % 16 == 0 and 0 < groups <= _lib.MAX_GROUPS
+            and bool(_lib.lib().dsl_gemm_kn_served(op, M, N, K, groups)))
+
+
 # --------------------------------------------------------------------------------------
 # low-level launches on already-quantised operands
 # --------------------------------------------------------------------------------------
@@ -149,20 +157,21 @@ def _offsets_arg(offsets: Optional[torch.Tensor], dev) -> Tuple[Optional[torch.T
 def gemm_fp8_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, scale_a: Scalar, scale_b: Scalar, *, n: int,
                        out_dtype=torch.float32, expert_offsets: Optional[torch.Tensor] = None,
                        row_scale=None, col_scale=None, b_static: bool = False, activation: Optional[str] = None,
-                       out_global_scale: Scalar = None):
-    """C = (qa @ qb^T) * scale_a * scale_b on E4M3 bytes; qa [M, K], qb_nk [G*N, K].
+                       out_global_scale: Scalar = None, b_kn: bool = False):
+    """C = (qa @ qb^T) * scale_a * scale_b on E4M3 bytes; qa [M, K], qb_nk [G*N, K] (`b_kn`: [G*K, N], read as it is).
     `b_static`: the weight was complete before the previous kernel on this stream was launched
     (lets the decode kernel stream it while the activation quantiser still runs)."""
     dev = _lib.require_cuda(qa, qb_nk)
     qa, qb_nk = _bytes2d(qa), _bytes2d(qb_nk)
     M, K = qa.shape
     offs, groups = _offsets_arg(expert_offsets, dev)
-    if qb_nk.shape != (groups * n, K):
+    if qb_nk.shape != ((groups * K, n) if b_kn else (groups * n, K)):
         raise ValueError(f"weight must be [{groups}*{n}, {K}] K-major bytes, got {tuple(qb_nk.shape)}")
     nc = _out_cols(n, activation)
     keep: list = []
     ep = _epilogue(dev, scale_a, scale_b, None, row_scale, col_scale, keep, b_static, activation,
                    (_lib.OP_GEMM_FP8, M, n, K, groups))
+    ep.b_is_kn = 1 if b_kn else 0
     out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
     with torch.cuda.device(dev):
         rc = _lib.lib().dsl_gemm_fp8(qa.data_ptr(), qb_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
@@ -174,7 +183,8 @@ def gemm_fp8_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, scale_a: Scalar, s
 def gemm_fp8_groupwise_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor, *,
                                  n: int, sb_block: bool, out_dtype=torch.float32,
                                  expert_offsets: Optional[torch.Tensor] = None,
-                                 row_scale=None, col_scale=None, activation: Optional[str] = None) -> torch.Tensor:
+                                 row_scale=None, col_scale=None, activation: Optional[str] = None,
+                                 b_kn: bool = False) -> torch.Tensor:
     """C = sum_g (qa_g @ qb_g^T) * sa[:, g] * sb[g]; sa [M, K/128]; sb [G, K/128, N] per-column
     (sb_block False, the layout of cuda/gemm/fp8_gemm.cu:75) or [G, ceil(N/128), K/128] blocks."""
     dev = _lib.require_cuda(qa, qb_nk, sa, sb)
@@ -183,7 +193,7 @@ def gemm_fp8_groupwise_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, sa: torc
     if K % 128 != 0:
         raise ValueError(f"K must be a multiple of 128 for group-scaled FP8, got {K}")
     offs, groups = _offsets_arg(expert_offsets, dev)
-    if qb_nk.shape != (groups * n, K):
+    if qb_nk.shape != ((groups * K, n) if b_kn else (groups * n, K)):
         raise ValueError(f"weight must be [{groups}*{n}, {K}] K-major bytes, got {tuple(qb_nk.shape)}")
     sa = sa.to(torch.float32).contiguous()
     sb = sb.to(torch.float32).contiguous()
@@ -199,6 +209,7 @@ def gemm_fp8_groupwise_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, sa: torc
     keep: list = []
     ep = _epilogue(dev, None, None, out.dtype, row_scale, col_scale, keep, False, activation,
                    (_lib.OP_GEMM_FP8_GROUPWISE, M, n, K, groups))
+    ep.b_is_kn = 1 if b_kn else 0
     with torch.cuda.device(dev):
         rc = _lib.lib().dsl_gemm_fp8_groupwise(qa.data_ptr(), qb_nk.data_ptr(), sa.data_ptr(), sb.data_ptr(),
                                                1 if sb_block else 0, out.data_ptr(), nc, M, n, K, _lib.ptr(offs),
@@ -254,17 +265,18 @@ def gemm_fp4_quantized(pa: torch.Tensor, pb_nk: torch.Tensor, sfa: torch.Tensor,
 
 def gemm_bf16_raw(a: torch.Tensor, b_nk: torch.Tensor, *, n: int, out_dtype=torch.float32,
                   expert_offsets: Optional[torch.Tensor] = None, scale_a: Scalar = None,
-                  scale_b: Scalar = None, activation: Optional[str] = None, out_global_scale: Scalar = None):
+                  scale_b: Scalar = None, activation: Optional[str] = None, out_global_scale: Scalar = None, b_kn: bool = False):
     dev = _lib.require_cuda(a, b_nk)
     a = a.to(torch.bfloat16).contiguous()
     b_nk = b_nk.to(torch.bfloat16).contiguous()
     M, K = a.shape
     offs, groups = _offsets_arg(expert_offsets, dev)
-    if b_nk.shape != (groups * n, K):
+    if b_nk.shape != ((groups * K, n) if b_kn else (groups * n, K)):
         raise ValueError(f"weight must be [{groups}*{n}, {K}] K-major, got {tuple(b_nk.shape)}")
     nc = _out_cols(n, activation)
     keep: list = []
     ep = _epilogue(dev, scale_a, scale_b, None, None, None, keep, False, activation, (_lib.OP_GEMM_BF16, M, n, K, groups))
+    ep.b_is_kn = 1 if b_kn else 0
     out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
     with torch.cuda.device(dev):
         rc = _lib.lib().dsl_gemm_bf16(a.data_ptr(), b_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
@@ -469,13 +481,14 @@ def fp8_gemm(A: torch.Tensor, B, scale_a: Scalar = None, scale_b: Scalar = None,
         raise TypeError("A and B must both be E4M3 bytes or both be high-precision")
     if a_q:
         qb = _bytes2d(B)
-        if b_layout == "kn":
+        b_kn = b_layout == "kn" and _kn_direct(_lib.OP_GEMM_FP8 if mode == "per_tensor" else _lib.OP_GEMM_FP8_GROUPWISE, qb, M)
+        if b_layout == "kn" and not b_kn:
             qb = transpose_bytes(qb)
         if mode == "per_tensor":
             if scale_a is None or scale_b is None:
                 raise ValueError("scale_a and scale_b are required for already-quantised operands")
             return gemm_fp8_quantized(A, qb, scale_a, scale_b, n=N, out_dtype=out_dtype, row_scale=row_scale,
-                                      col_scale=col_scale)
+                                      col_scale=col_scale, b_kn=b_kn)
         if not isinstance(scale_a, torch.Tensor) or not isinstance(scale_b, torch.Tensor):
             raise TypeError("group-scaled FP8 needs scale_a and scale_b tensors")
         if group_size != 128:
@@ -490,7 +503,7 @@ def fp8_gemm(A: torch.Tensor, B, scale_a: Scalar = None, scale_b: Scalar = None,
             scale_b = (scale_b.repeat_interleave(rep, dim=1)[:, :kg] if mode == "block128"
                        else scale_b.repeat_interleave(rep, dim=0)[:kg]).contiguous()
         return gemm_fp8_groupwise_quantized(A, qb, scale_a, scale_b, n=N, sb_block=(mode == "block128"),
-                                            out_dtype=out_dtype, row_scale=row_scale, col_scale=col_scale)
+                                            out_dtype=out_dtype, row_scale=row_scale, col_scale=col_scale, b_kn=b_kn)
     if A.dtype not in _FLOAT_DTYPES or B.dtype not in _FLOAT_DTYPES:
         raise TypeError(f"unsupported dtypes {A.dtype}, {B.dtype}")
     if mode != "per_tensor" and group_size != 128:
@@ -617,16 +630,19 @@ def grouped_gemm(A: torch.Tensor, B, num_groups: Optional[int] = None, expert_of
     fixed = A.dim() == 3
     if not fixed and (A.dim() != 2 or expert_offsets is None):
         raise ValueError("A must be [G,M,K], or [sum M, K] together with expert_offsets")
+    w = None
     if isinstance(B, PackedWeight):
         w = B
         if w.format != formats[format]:
             raise ValueError(f"packed weight is {w.format}, need {formats[format]}")
-    else:
-        if B.dim() != 3:
-            raise ValueError(f"B must be 3-D, got {tuple(B.shape)}")
+    elif B.dim() != 3:
+        raise ValueError(f"B must be 3-D, got {tuple(B.shape)}")
+    elif not (format == "bf16" and b_layout == "kn" and not glu and not cache_weights and B.dtype == torch.bfloat16
+              and A.dtype in _FLOAT_DTYPES and A.shape[-1] == B.shape[1]
+              and _kn_direct(_lib.OP_GEMM_BF16, B, A.numel() // max(A.shape[-1], 1), B.shape[0])):
         w = (cached_pack(B, formats[format], b_layout, gate_up_interleave=glu) if cache_weights
              else pack_weight(B, formats[format], layout=b_layout, gate_up_interleave=glu))
-    G = w.groups
+    G = B.shape[0] if w is None else w.groups
     if num_groups is not None and int(num_groups) != G:
         raise ValueError(f"num_groups={num_groups} but B holds {G} groups")
     if fixed:
@@ -634,7 +650,8 @@ def grouped_gemm(A: torch.Tensor, B, num_groups: Optional[int] = None, expert_of
             raise ValueError(f"A holds {A.shape[0]} groups but B holds {G}")
         Mg = A.shape[1]
         a2 = A.reshape(G * Mg, A.shape[2])
-        offs = torch.arange(G + 1, dtype=torch.int32, device=dev) * Mg
+        offs = (torch.arange(0, G * Mg + 1, Mg, dtype=torch.int32, device=dev) if Mg > 0
+                else torch.zeros(G + 1, dtype=torch.int32, device=dev))
     else:
         a2 = A
         offs = expert_offsets
@@ -644,11 +661,17 @@ def grouped_gemm(A: torch.Tensor, B, num_groups: Optional[int] = None, expert_of
         out_dtype = A.dtype if (format == "bf16" and A.dtype in (torch.float32, torch.bfloat16)) else torch.float32
     if G == 1:
         offs = None
-    out = linear(a2.contiguous(), w, out_dtype=out_dtype, expert_offsets=offs, activation=activation)
+    if w is None:
+        out = gemm_bf16_raw(a2, B.reshape(G * B.shape[1], B.shape[2]), n=B.shape[2], out_dtype=out_dtype, expert_offsets=offs, b_kn=True)
+    else:
+        out = linear(a2.contiguous(), w, out_dtype=out_dtype, expert_offsets=offs, activation=activation)
     return out.reshape(G, Mg, out.shape[1]) if fixed else out
 
 
 def bf16_gemm(A: torch.Tensor, B: torch.Tensor, *, b_layout: str = "kn", out_dtype="float32") -> torch.Tensor:
     """BF16 GEMM with fp32 accumulation, C = A[M,K] @ B[K,N] -> fp32 (triton/gemm/gemm_kernels.py:49-65)."""
+    if (b_layout == "kn" and A.dim() == 2 and B.dim() == 2 and A.shape[1] == B.shape[0] and A.is_cuda and B.device == A.device
+            and A.dtype in _FLOAT_DTYPES and B.dtype == torch.bfloat16 and _kn_direct(_lib.OP_GEMM_BF16, B, A.shape[0])):
+        return gemm_bf16_raw(A, B, n=B.shape[1], out_dtype=out_dtype, b_kn=True)
     w = pack_weight(B, "bf16", layout=b_layout)
     return linear(A, w, out_dtype=out_dtype)

@@ -158,7 +158,15 @@ typedef struct {
     int act_scale_per_token;    /* dsl_linear with an NVFP4 weight only: quantise the activations with per-token global
                                    scales (dsl_quant_fp4_per_token, one pass) and apply them as the per-token rescale;
                                    row_scale must then be NULL */
+    int b_is_kn;                /* dsl_gemm_fp8, dsl_gemm_bf16 and dsl_gemm_fp8_groupwise: B is given [K, N] / [G, K, N]
+                                   (the reference's layout, cuda/gemm/fp8_gemm.cu:29-35) and the tensor cores read it as
+                                   it is; only for problems dsl_gemm_kn_served says yes to, else DSL_ERR_SHAPE */
 } dsl_epilogue;
+
+/* Whether the GEMM entry point `op` (DSL_OP_*) takes B as [K, N] for this problem, given the workspace that
+ * dsl_workspace_bytes asks for: FP8 and BF16 operands with N a multiple of 16 bytes, in the shapes the CTA-pair kernels
+ * (M > 128, N >= 256) and the weight-streaming kernel serve. */
+int dsl_gemm_kn_served(int op, long long M, int N, int K, int groups);
 
 /*
  * Bytes of dsl_epilogue.workspace that the GEMM entry point `op` can put to use for a dense M x N x K
