@@ -294,15 +294,20 @@ _OP_OF_FORMAT = {"fp8": _lib.OP_GEMM_FP8, "fp8_block128": _lib.OP_GEMM_FP8_GROUP
                  "mxfp4": _lib.OP_GEMM_FP4_MX, "bf16": _lib.OP_GEMM_BF16}
 
 
+def _new_weight_desc(w: PackedWeight) -> "_lib.Weight":
+    d = _lib.Weight()
+    d.format, d.groups, d.n, d.k = _W_CODES[w.format], w.groups, w.n, w.k
+    d.q = w.q.data_ptr()
+    d.scale = None if w.scale is None else w.scale.data_ptr()
+    d.global_scale = None if w.global_scale is None else w.global_scale.data_ptr()
+    return d
+
+
 def _weight_desc(w: PackedWeight) -> "_lib.Weight":
     """The weight's dsl_weight struct, built once and kept on the PackedWeight (rebuilt if its tensors were swapped)."""
     d = getattr(w, "_cdesc", None)
     if d is None or d.q != w.q.data_ptr():
-        d = _lib.Weight()
-        d.format, d.groups, d.n, d.k = _W_CODES[w.format], w.groups, w.n, w.k
-        d.q = w.q.data_ptr()
-        d.scale = None if w.scale is None else w.scale.data_ptr()
-        d.global_scale = None if w.global_scale is None else w.global_scale.data_ptr()
+        d = _new_weight_desc(w)
         w._cdesc = d
         w._scratch_need = {}
     return d

@@ -24,13 +24,14 @@ Expert parallelism, two ways (`moe_forward(..., dispatch=...)`):
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
 import torch
 
 from . import _lib
-from .gemm_kernels import gemm_fp4_quantized, gemm_fp8_groupwise_quantized, gemm_fp8_quantized, linear
+from .gemm_kernels import _new_weight_desc, gemm_fp4_quantized, gemm_fp8_groupwise_quantized, gemm_fp8_quantized, linear
 from .quantize import PackedWeight, pack_weight, quantize_fp4, quantize_fp8
 from .sharding import arrival_expert_ids, exchange_rows, expert_ranges, return_rows
 
@@ -191,6 +192,44 @@ def _experts_fp4(p: MoEPlan, packed: torch.Tensor, sf: torch.Tensor, gs, w: MoEW
                               global_scale_b=w.down.global_scale, out_dtype=torch.bfloat16, **common)
 
 
+def _whole_layer(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, renormalize: bool, out_dtype,
+                 act_global_scale) -> Optional[torch.Tensor]:
+    """The layer through the single C entry point `dsl_moe_layer` (same launches, same bits as the steps below, without
+    the host time between them), or None when that call does not take it: only part of the experts, shapes the packed
+    weights do not match, row lengths its dispatch cannot move."""
+    gu, dn, hgs = w.gate_up, w.down, w.hidden_global_scale
+    if (w.first != 0 or w.last != w.experts or gu.groups != w.experts or dn.groups != w.experts or gu.format != dn.format
+            or x.dim() != 2 or logits.dim() != 2 or logits.shape != (x.shape[0], w.experts) or x.shape[0] == 0 or x.shape[1] != gu.k
+            or logits.dtype not in (torch.float32, torch.bfloat16) or x.dtype not in (torch.float32, torch.bfloat16, torch.float16)
+            or out_dtype not in (torch.float32, torch.bfloat16) or not 1 <= k <= min(32, w.experts)):
+        return None
+    fused = gu.format == "nvfp4" and hgs is not None
+    if (fused and (isinstance(hgs, torch.Tensor) or not hgs > 0)) or isinstance(act_global_scale, str):
+        return None
+    dev = _lib.require_cuda(x, logits, gu.q, dn.q)
+    lib = _lib.lib()
+    x = x.to(torch.bfloat16).contiguous() if gu.format == "bf16" else x.contiguous()
+    logits = logits.contiguous()
+    act_gs = None
+    if gu.format == "nvfp4" and act_global_scale is not None:
+        act_gs = (act_global_scale.detach().to(device=dev, dtype=torch.float32).reshape(1) if isinstance(act_global_scale, torch.Tensor)
+                  else torch.full((1,), float(act_global_scale), dtype=torch.float32, device=dev))
+    du, dd = _new_weight_desc(gu), _new_weight_desc(dn)
+    T = x.shape[0]
+    need = int(lib.dsl_moe_layer_scratch_bytes(ctypes.byref(du), ctypes.byref(dd), T, k, 1 if fused else 0))
+    if need == 0:
+        return None
+    with torch.cuda.device(dev):
+        scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+        out = torch.empty((T, dn.n), dtype=out_dtype, device=dev)
+        rc = lib.dsl_moe_layer(x.data_ptr(), _lib.dtype_code(x.dtype), logits.data_ptr(), _lib.dtype_code(logits.dtype), T, k,
+                               1 if renormalize else 0, ctypes.byref(du), ctypes.byref(dd), _lib.ptr(act_gs), 1 if fused else 0,
+                               float(hgs) if fused else 1.0, scratch.data_ptr(), need, out.data_ptr(), _lib.dtype_code(out_dtype),
+                               _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+    _lib.check(rc, "dsl_moe_layer")
+    return out
+
+
 def moe_partial(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, *, renormalize: bool = True,
                 out_dtype=torch.float32, act_global_scale=None, out=None) -> torch.Tensor:
     """This rank's share of the layer's result, [tokens, D] (fp32, or bf16 = the fp32 sum rounded once, which saves
@@ -201,6 +240,10 @@ def moe_partial(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, *,
     the host once).  `act_global_scale` (NVFP4: a number or a one-element tensor) is a calibrated global scale of x;
     the quantiser then makes ONE pass over x instead of an amax pass and a quantise pass."""
     fmt = w.gate_up.format
+    if out is None:
+        whole = _whole_layer(x, logits, w, k, renormalize, out_dtype, act_global_scale)
+        if whole is not None:
+            return whole
     ids, wts = route(logits, k, renormalize)
     p = plan(ids, wts, w.experts)
     offs = _local_offsets(p, w.first, w.last)

@@ -303,6 +303,21 @@ int dsl_moe_dispatch_rows(const void* x, const int* ids, const int* dest, const 
 int dsl_moe_combine(const void* y, int y_dtype, const int* ids, const int* dest, const int* offsets, const float* weights,
                     int tokens, int k, int d_model, int first_expert, int last_expert, void* out, int out_dtype,
                     void* stream);
+/*
+ * The whole layer on a GPU that holds every expert, in one call: route, plan, quantise the tokens, dispatch, gate/up GEMM
+ * with SwiGLU, down GEMM, combine - the steps above and the GEMM entry points, in that order, with every intermediate in
+ * `scratch` (256-byte aligned, dsl_moe_layer_scratch_bytes; consumed within the call, so calls issued in order on one stream
+ * may share it).  gate_up is [experts, 2H, K] with its rows interleaved, down [experts, D, H], both of one format; K and H
+ * as the format's quantiser and GEMM need them, 128x128 FP8 also K % 512 == 0 (scale rows are dispatched as 16-byte
+ * vectors); dsl_moe_layer_scratch_bytes returns 0 for what the call does not take.
+ *   act_gs_dev    NVFP4: calibrated global scale of x (device float), or NULL: amax / 2688
+ *   fused_hidden  NVFP4: quantise the hidden activation in the gate/up GEMM with the global scale hidden_gs
+ */
+size_t dsl_moe_layer_scratch_bytes(const dsl_weight* gate_up, const dsl_weight* down, int tokens, int k, int fused_hidden);
+int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int logits_dtype, int tokens, int k, int renorm,
+                  const dsl_weight* gate_up, const dsl_weight* down, const float* act_gs_dev, int fused_hidden,
+                  float hidden_gs, void* scratch, size_t scratch_bytes, void* out, int out_dtype, uint32_t* status,
+                  void* stream);
 size_t dsl_moe_wire_bytes(int K, int format);
 /*
  * Sum of the ranks' partial results over peer memory (expert-parallel layer whose ranks keep their own token rows; no

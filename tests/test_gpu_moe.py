@@ -256,3 +256,24 @@ def test_combine_slot_batches(cuda_device, k, Dm, y_dtype, out_dtype):
     want = terms.sum(1)
     bound = (k + 1) * 2.0 ** -24 * terms.abs().sum(1) + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
     assert bool(((got.double() - want).abs() <= bound + 1e-30).all())
+
+
+# The one-call layer against the step-by-step form (which expert-parallel ranks use), bit for bit: every format, fused and
+# separate hidden quantisation, both logits dtypes, row lengths whose scale tiles are partly padding, one token, one expert.
+@pytest.mark.parametrize("fmt,hgs", [("nvfp4", 0.004), ("nvfp4", None), ("mxfp4", None), ("fp8", None), ("fp8_block128", None), ("bf16", None)])
+@pytest.mark.parametrize("T,E,k,K,H,Dm", [(96, 6, 2, 512, 128, 192), (1, 5, 3, 512, 256, 256), (40, 1, 1, 512, 128, 272), (700, 9, 4, 1024, 384, 520),
+                                          (33, 7, 2, 672, 224, 128)])
+def test_one_call_layer_equals_the_steps(cuda_device, monkeypatch, fmt, hgs, T, E, k, K, H, Dm):
+    if fmt == "fp8_block128" and K % 128:
+        pytest.skip("K % 128")
+    rng = np.random.default_rng(T + K)
+    x, logits, w1, w2 = _layer_inputs(rng, T, E, K, H, Dm, cuda_device)
+    wts = D.MoEWeights.pack(w1, w2, fmt, hidden_global_scale=hgs)
+    for lg, out_dtype, gs in ((logits, torch.bfloat16, None), (logits.bfloat16(), torch.float32, 0.002 if fmt == "nvfp4" else None)):
+        assert moe._whole_layer(x, lg, wts, k, True, out_dtype, gs) is not None
+        got = D.moe_forward(x, lg, wts, k, out_dtype=out_dtype, act_global_scale=gs)
+        _lib.check_status()
+        with monkeypatch.context() as m:
+            m.setattr(moe, "_whole_layer", lambda *a: None)
+            want = D.moe_forward(x, lg, wts, k, out_dtype=out_dtype, act_global_scale=gs)
+        assert got.dtype == out_dtype and torch.equal(got, want)
