@@ -274,7 +274,10 @@ int dsl_gemm_kn_served(int op, long long M, int N, int K, int groups) {
     GemmArgs a;
     int kind;
     if (!problem_of(op, M, N, K, &kind, &a)) return 0;
-    if (groups > 1) a.group_offsets = reinterpret_cast<const int*>(uintptr_t(16));   // "row groups": never dereferenced
+    if (groups > 1) {
+        a.group_offsets = reinterpret_cast<const int*>(uintptr_t(16));   // "row groups": never dereferenced
+        a.num_groups = groups;
+    }
     return kn_served(kind, a) ? 1 : 0;
 }
 

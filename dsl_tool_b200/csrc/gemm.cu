@@ -536,14 +536,15 @@ bool kn_served(int kind, const GemmArgs& args) {
     if (args.n <= 0 || args.m_total <= 0 || (static_cast<long long>(args.n) * elem) % 16 != 0 || forced_kernel() != 0) return false;
     bool decode = false;
     decode_scratch_bytes(kind, args, &decode);
-    return decode || (args.m_total > 128 && args.n >= 256);
+    return decode || decode_grouped_served(args) || (args.m_total > 128 && args.n >= 256);
 }
 
 int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st) {
     if (args.m_total <= 0 || args.n <= 0) return 0;
     const int forced = forced_kernel();
     if (forced == 0 || forced == 3) {
-        const int rc = launch_gemm_decode(kind, A, B, args, st);
+        int rc = launch_gemm_decode(kind, A, B, args, st);
+        if (rc == DSL_NOT_SERVED) rc = launch_gemm_decode_grouped(kind, A, B, args, st);
         if (rc != DSL_NOT_SERVED) return rc;
     }
     if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) return launch_gemm_pair(kind, A, B, args, st);

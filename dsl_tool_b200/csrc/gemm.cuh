@@ -75,6 +75,9 @@ constexpr int DSL_DECODE_MAX_ROWS = 128;   // activation rows the weight-streami
 constexpr int DSL_NOT_SERVED = -1000;      // launch_gemm_decode: problem outside its domain, use the tiled kernels
 
 int launch_gemm_decode(int kind, const void* A, const void* B, const GemmArgs& args, cudaStream_t st);
+// Row groups of few rows each: the weight-streaming kernel of gemm_decode_grouped.cu, or DSL_NOT_SERVED.
+bool decode_grouped_served(const GemmArgs& args);
+int launch_gemm_decode_grouped(int kind, const void* A, const void* B, const GemmArgs& args, cudaStream_t st);
 // Scratch bytes (behind the header) the weight-streaming kernel would use for this problem; 0 when it
 // combines inside clusters or does not serve the problem (*served says which).
 size_t decode_scratch_bytes(int kind, const GemmArgs& args, bool* served);

@@ -39,6 +39,15 @@ __device__ __forceinline__ void store_nvfp4_block(const GemmArgs& args, int row,
         static_cast<uint8_t>(sfb);
 }
 
+// (gate, up) -> silu(gate) * up or gelu(gate) * up.  SwiGLU: silu(x) = x / (1 + exp(-x))
+// (cuda/activations/fused_gated_activations.cu:27-29).  GeGLU: gelu(x) = 0.5 x (1 + tanh(c (x + k x^3))) (:32-37)
+// = x / (1 + exp(-2c (x + k x^3))), the same shape.  Fast exponential and division (a few ulp): the epilogue must stay
+// shorter than a tile's MMAs.
+__device__ __forceinline__ float glu_value(bool geglu, float gate, float up) {
+    const float z = geglu ? 1.5957691216f * (gate + 0.044715f * gate * gate * gate) : gate;
+    return __fmul_rn(__fdividef(gate, 1.0f + __expf(-z)), up);
+}
+
 // v: 32 fp32 accumulators (bit patterns) of row `row`, columns col0..col0+31 of group `group`.
 // out = (acc * s1) * s2 [* row_scale[row]] [* col_scale[group*n + col]]
 // sf_tile / rin: only read when the result is quantised (args.out_sf != nullptr).
@@ -63,18 +72,11 @@ __device__ __forceinline__ void store_chunk32_t(const GemmArgs& args, int row, i
             if (col0 + i < args.n) f[i] = __fmul_rn(f[i], cs[col0 + i]);
     }
     if (FULL && args.act != DSL_ACT_NONE) {
-        // columns (2j, 2j+1) = (gate_j, up_j) -> output column col0/2 + j of an [m, n/2] result;
-        // SwiGLU: silu(x) = x / (1 + exp(-x)) (cuda/activations/fused_gated_activations.cu:27-29).
-        // GeGLU: gelu(x) = 0.5 x (1 + tanh(c (x + k x^3))) (:32-37) = x / (1 + exp(-2c (x + k x^3))), the same shape.
+        // columns (2j, 2j+1) = (gate_j, up_j) -> output column col0/2 + j of an [m, n/2] result
         const bool geglu = args.act == DSL_ACT_GEGLU;
         float o[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float g = f[2 * j];
-            const float z = geglu ? 1.5957691216f * (g + 0.044715f * g * g * g) : g;
-            // fast exponential and division (a few ulp): the epilogue must stay shorter than a tile's MMAs
-            o[j] = __fmul_rn(__fdividef(g, 1.0f + __expf(-z)), f[2 * j + 1]);
-        }
+        for (int j = 0; j < 16; ++j) o[j] = glu_value(geglu, f[2 * j], f[2 * j + 1]);
         const int c0 = col0 >> 1;
         if (args.out_sf != nullptr) {     // n/2 is a multiple of 16 here, so the 16 outputs are one whole block
             if (col0 < args.n) store_nvfp4_block(args, row, c0, o, args.out_gs_dev != nullptr ? *args.out_gs_dev : args.out_gs, sf_tile, rin);
