@@ -10,6 +10,59 @@ using namespace dsl;
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+namespace dsl {
+
+int quant_fp4_impl(const void* x, int dtype, long long rows, long long cols, int format, float* gs_io, int gs_given, uint8_t* q_out,
+                   uint8_t* sf_out, const int* group_offsets, int groups, void* ws, bool rows_unpadded, void* stream) {
+    if (x == nullptr || q_out == nullptr || sf_out == nullptr) return DSL_ERR_NULL;
+    if (dtype < DSL_F32 || dtype > DSL_F16) return DSL_ERR_ENUM;
+    if (format != DSL_FP4_NV && format != DSL_FP4_MX) return DSL_ERR_ENUM;
+    if (format == DSL_FP4_NV && gs_io == nullptr) return DSL_ERR_NULL;
+    if (format == DSL_FP4_NV && !gs_given && ws == nullptr) return DSL_ERR_NULL;
+    if (rows < 0 || cols < 0 || rows > (1ll << 31) || cols > (1ll << 31) || cols % 32 != 0) return DSL_ERR_SHAPE;
+    if (group_offsets != nullptr && (groups < 1 || groups > DSL_MAX_GROUPS)) return DSL_ERR_TOO_LARGE;
+    if (!aligned16(x) || !aligned16(q_out) || !aligned16(sf_out)) return DSL_ERR_ALIGN;
+    if (rows == 0 || cols == 0) return 0;
+    const long long nblk = format == DSL_FP4_NV ? cols / 16 : cols / 32;
+    size_t sf_bytes;
+    int clear;
+    if (group_offsets != nullptr) {
+        sf_bytes = dsl_sf_bytes_grouped(rows, nblk, groups);
+        clear = rows_unpadded ? nblk % 4 != 0 : 1;
+    } else {
+        sf_bytes = dsl_sf_bytes(rows, nblk);
+        clear = ((rows % 128 != 0 && !rows_unpadded) || nblk % 4 != 0) ? 1 : 0;   // padding bytes must read as zero
+    }
+    return static_cast<int>(launch_quant_fp4(x, dtype, rows, cols, format, gs_io, gs_given, q_out, sf_out, sf_bytes,
+                                             clear, group_offsets, groups, static_cast<uint32_t*>(ws),
+                                             as_stream(stream)));
+}
+
+int quant_fp4_per_token_impl(const void* x, int dtype, long long rows, long long cols, float* gs_out, uint8_t* q_out, uint8_t* sf_out,
+                             const int* group_offsets, int groups, bool rows_unpadded, void* stream) {
+    if (x == nullptr || q_out == nullptr || sf_out == nullptr || gs_out == nullptr) return DSL_ERR_NULL;
+    if (dtype < DSL_F32 || dtype > DSL_F16) return DSL_ERR_ENUM;
+    if (rows < 0 || cols < 0 || rows > (1ll << 31) || cols % 32 != 0) return DSL_ERR_SHAPE;
+    if (cols > DSL_PER_TOKEN_MAX_COLS) return DSL_ERR_TOO_LARGE;      // a row is held in one CTA's registers
+    if (group_offsets != nullptr && (groups < 1 || groups > DSL_MAX_GROUPS)) return DSL_ERR_TOO_LARGE;
+    if (!aligned16(x) || !aligned16(q_out) || !aligned16(sf_out)) return DSL_ERR_ALIGN;
+    if (rows == 0 || cols == 0) return 0;
+    const long long nblk = cols / 16;
+    size_t sf_bytes;
+    int clear;
+    if (group_offsets != nullptr) {
+        sf_bytes = dsl_sf_bytes_grouped(rows, nblk, groups);
+        clear = rows_unpadded ? nblk % 4 != 0 : 1;
+    } else {
+        sf_bytes = dsl_sf_bytes(rows, nblk);
+        clear = ((rows % 128 != 0 && !rows_unpadded) || nblk % 4 != 0) ? 1 : 0;
+    }
+    return static_cast<int>(launch_quant_nvfp4_per_token(x, dtype, rows, cols, gs_out, q_out, sf_out, sf_bytes, clear, group_offsets,
+                                                         groups, as_stream(stream)));
+}
+
+}  // namespace dsl
+
 extern "C" {
 
 const char* dsl_version(void) { return "dslgemm 0.1 (sm_100a)"; }
@@ -41,51 +94,12 @@ int dsl_quant_fp8(const void* x, int dtype, long long rows, long long cols, int 
 int dsl_quant_fp4(const void* x, int dtype, long long rows, long long cols, int format, float* gs_io,
                   int gs_given, uint8_t* q_out, uint8_t* sf_out, const int* group_offsets, int groups,
                   void* ws, void* stream) {
-    if (x == nullptr || q_out == nullptr || sf_out == nullptr) return DSL_ERR_NULL;
-    if (dtype < DSL_F32 || dtype > DSL_F16) return DSL_ERR_ENUM;
-    if (format != DSL_FP4_NV && format != DSL_FP4_MX) return DSL_ERR_ENUM;
-    if (format == DSL_FP4_NV && gs_io == nullptr) return DSL_ERR_NULL;
-    if (format == DSL_FP4_NV && !gs_given && ws == nullptr) return DSL_ERR_NULL;
-    if (rows < 0 || cols < 0 || rows > (1ll << 31) || cols > (1ll << 31) || cols % 32 != 0) return DSL_ERR_SHAPE;
-    if (group_offsets != nullptr && (groups < 1 || groups > DSL_MAX_GROUPS)) return DSL_ERR_TOO_LARGE;
-    if (!aligned16(x) || !aligned16(q_out) || !aligned16(sf_out)) return DSL_ERR_ALIGN;
-    if (rows == 0 || cols == 0) return 0;
-    const long long nblk = format == DSL_FP4_NV ? cols / 16 : cols / 32;
-    size_t sf_bytes;
-    int clear;
-    if (group_offsets != nullptr) {
-        sf_bytes = dsl_sf_bytes_grouped(rows, nblk, groups);
-        clear = 1;
-    } else {
-        sf_bytes = dsl_sf_bytes(rows, nblk);
-        clear = (rows % 128 != 0 || nblk % 4 != 0) ? 1 : 0;   // padding bytes must read as zero
-    }
-    return static_cast<int>(launch_quant_fp4(x, dtype, rows, cols, format, gs_io, gs_given, q_out, sf_out, sf_bytes,
-                                             clear, group_offsets, groups, static_cast<uint32_t*>(ws),
-                                             as_stream(stream)));
+    return quant_fp4_impl(x, dtype, rows, cols, format, gs_io, gs_given, q_out, sf_out, group_offsets, groups, ws, false, stream);
 }
 
 int dsl_quant_fp4_per_token(const void* x, int dtype, long long rows, long long cols, float* gs_out, uint8_t* q_out,
                             uint8_t* sf_out, const int* group_offsets, int groups, void* stream) {
-    if (x == nullptr || q_out == nullptr || sf_out == nullptr || gs_out == nullptr) return DSL_ERR_NULL;
-    if (dtype < DSL_F32 || dtype > DSL_F16) return DSL_ERR_ENUM;
-    if (rows < 0 || cols < 0 || rows > (1ll << 31) || cols % 32 != 0) return DSL_ERR_SHAPE;
-    if (cols > DSL_PER_TOKEN_MAX_COLS) return DSL_ERR_TOO_LARGE;      // a row is held in one CTA's registers
-    if (group_offsets != nullptr && (groups < 1 || groups > DSL_MAX_GROUPS)) return DSL_ERR_TOO_LARGE;
-    if (!aligned16(x) || !aligned16(q_out) || !aligned16(sf_out)) return DSL_ERR_ALIGN;
-    if (rows == 0 || cols == 0) return 0;
-    const long long nblk = cols / 16;
-    size_t sf_bytes;
-    int clear;
-    if (group_offsets != nullptr) {
-        sf_bytes = dsl_sf_bytes_grouped(rows, nblk, groups);
-        clear = 1;
-    } else {
-        sf_bytes = dsl_sf_bytes(rows, nblk);
-        clear = (rows % 128 != 0 || nblk % 4 != 0) ? 1 : 0;
-    }
-    return static_cast<int>(launch_quant_nvfp4_per_token(x, dtype, rows, cols, gs_out, q_out, sf_out, sf_bytes, clear, group_offsets,
-                                                         groups, as_stream(stream)));
+    return quant_fp4_per_token_impl(x, dtype, rows, cols, gs_out, q_out, sf_out, group_offsets, groups, false, stream);
 }
 
 int dsl_pack_kn(const void* w, int dtype, int groups, int K, int N, int format, int interleave, float* scale_io, int scale_given,

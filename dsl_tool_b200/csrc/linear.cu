@@ -10,6 +10,10 @@
 #include <cuda_runtime.h>
 
 #include "dslgemm.h"
+#include "quant.cuh"
+
+using dsl::quant_fp4_impl;
+using dsl::quant_fp4_per_token_impl;
 
 namespace {
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -98,13 +102,16 @@ extern "C" int dsl_linear(const void* x, int x_dtype, long long M, const dsl_wei
             if (w->scale == nullptr) return DSL_ERR_NULL;
             const int fmt = w->format == DSL_W_NVFP4 ? DSL_FP4_NV : DSL_FP4_MX;
             if (fmt == DSL_FP4_NV && w->global_scale == nullptr) return DSL_ERR_NULL;
+            // The scale bytes of a tile's missing rows stay unwritten (they reach only result rows that nobody stores):
+            // one launch less (24 x 28672 x 8192 MXFP4: 34.8 -> 30.7 us a call; 1 x 8192 x 8192 NVFP4: 20.8 -> 19.5 us).
+            constexpr bool rows_unpadded = true;
             // NVFP4: a global scale handed in through ep->scale_a_dev (calibrated, or known from the producer of x)
             // is used as it is, which makes the quantiser ONE pass over x; otherwise it comes from an amax pass
             if (ep->act_scale_per_token) {
                 if (fmt != DSL_FP4_NV) return DSL_ERR_ENUM;
                 if (ep->row_scale != nullptr) return DSL_ERR_ENUM;      // the per-token factor occupies that slot
                 float* gs_rows = reinterpret_cast<float*>(base + c.off_rows);
-                rc = dsl_quant_fp4_per_token(x, x_dtype, M, w->k, gs_rows, qa, static_cast<uint8_t*>(scales), offs, w->groups, stream);
+                rc = quant_fp4_per_token_impl(x, x_dtype, M, w->k, gs_rows, qa, static_cast<uint8_t*>(scales), offs, w->groups, rows_unpadded, stream);
                 if (rc != 0) return rc;
                 e.scale_a_dev = nullptr;
                 e.scale_a_host = 1.0f;
@@ -116,8 +123,8 @@ extern "C" int dsl_linear(const void* x, int x_dtype, long long M, const dsl_wei
             }
             const bool gs_given = fmt == DSL_FP4_NV && ep->scale_a_dev != nullptr;
             float* gs_io = gs_given ? const_cast<float*>(ep->scale_a_dev) : gs;
-            rc = dsl_quant_fp4(x, x_dtype, M, w->k, fmt, gs_io, gs_given ? 1 : 0, qa, static_cast<uint8_t*>(scales), offs, w->groups,
-                               ws, stream);
+            rc = quant_fp4_impl(x, x_dtype, M, w->k, fmt, gs_io, gs_given ? 1 : 0, qa, static_cast<uint8_t*>(scales), offs, w->groups,
+                                ws, rows_unpadded, stream);
             if (rc != 0) return rc;
             if (fmt == DSL_FP4_NV) {
                 e.scale_a_dev = gs_io;

@@ -138,3 +138,50 @@ def test_group_scaled_fp8(cuda_device, sb_block, M, N, K):
     assert torch.equal(got, gemm_fp8_groupwise_quantized(*args, n=N, sb_block=sb_block))
     scaled = gemm_fp8_groupwise_quantized(*args, n=N, sb_block=sb_block, out_dtype="bfloat16", row_scale=sa[:, 0], col_scale=col)
     assert torch.equal(scaled, (got * sa[:, :1] * col).bfloat16())
+
+
+# The fused gated activation in the streaming kernel, for every way of cutting the work (clusters of 4 and of 2, whole tiles,
+# runs across tiles) and ragged edges, against the activation of the kernel's own fp32 product.  The epilogue's exponential
+# and division are good to a few ulp (2^-22), relative to the result: 1e-6 in the norm.
+@pytest.mark.parametrize("activation", ["swiglu", "geglu"])
+@pytest.mark.parametrize("fmt", ["nvfp4", "fp8", "fp8_block128", "bf16"])
+@pytest.mark.parametrize("N,K,M", [(2304, 4096, 16), (6400, 1024, 33), (12800, 512, 9), (19200, 1024, 30), (1004, 1152, 100), (2304, 1152, 128)])
+def test_gated_activation(cuda_device, fmt, N, K, M, activation):
+    from dsl_tool_b200 import _lib, pack_weight
+    from dsl_tool_b200.gemm_kernels import linear
+    gen = torch.Generator(device="cuda").manual_seed(N + M)
+    a = torch.randn((M, K), generator=gen, device="cuda").bfloat16()
+    w = pack_weight((torch.randn((N, K), generator=gen, device="cuda") * 0.05).bfloat16(), fmt, gate_up_interleave=True)
+    col, row = torch.rand(N, generator=gen, device="cuda") + 0.5, torch.rand(M, generator=gen, device="cuda") + 0.5
+    x = linear(a, w, row_scale=row, col_scale=col).double()
+    gate, up = x[:, 0::2], x[:, 1::2]
+    act = torch.nn.functional.silu(gate) if activation == "swiglu" else torch.nn.functional.gelu(gate, approximate="tanh")
+    got = linear(a, w, row_scale=row, col_scale=col, activation=activation)
+    _lib.check_status()
+    assert got.shape == (M, N // 2)
+    assert float((got - act * up).norm() / (act * up).norm()) <= 1e-6
+    assert torch.equal(linear(a, w, row_scale=row, col_scale=col, activation=activation, out_dtype="bfloat16"), got.bfloat16())
+
+
+# Scale bytes of activation rows that do not exist are left as they are in the scratch of a linear() call: whatever lies
+# there (here NaN patterns), the result is that of a clean scratch.  Streaming and tiled kernels, scale tiles that end
+# inside a K block and that do not, row groups.
+@pytest.mark.parametrize("fmt,scale", [("nvfp4", None), ("nvfp4", 0.002), ("nvfp4", "per_token"), ("mxfp4", None)])
+@pytest.mark.parametrize("M,N,K,groups", [(3, 512, 1024, 1), (40, 512, 1056, 1), (200, 512, 1024, 1), (200, 100, 1056, 1), (90, 256, 512, 3),
+                                          (300, 256, 1056, 3)])
+def test_scratch_contents_do_not_matter(cuda_device, fmt, scale, M, N, K, groups):
+    from dsl_tool_b200 import _lib, pack_weight
+    from dsl_tool_b200.gemm_kernels import linear
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    a = torch.randn((M, K), generator=gen, device="cuda").bfloat16()
+    shape = (N, K) if groups == 1 else (groups, N, K)
+    w = pack_weight((torch.randn(shape, generator=gen, device="cuda") * 0.05).bfloat16(), fmt)
+    offs = None if groups == 1 else torch.tensor([0, M // 5, M // 5, M], dtype=torch.int32, device="cuda")
+    results = []
+    for fill in (0, 255):
+        linear(a, w, expert_offsets=offs, act_global_scale=scale)
+        buf = _lib.act_arena(a.device, torch.cuda.current_stream().cuda_stream).buf
+        buf.fill_(fill)
+        results.append(linear(a, w, expert_offsets=offs, act_global_scale=scale))
+    _lib.check_status()
+    assert torch.equal(results[0], results[1]) and bool(results[0].isfinite().all())
