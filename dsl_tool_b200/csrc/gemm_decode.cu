@@ -25,6 +25,8 @@
 //     columns: 16 x 4096 x 14336 with 128x128 block scales took 73.0 us per call (quantiser included), 19.6 us here,
 //     the kernel alone 16.1 us = 3.6 TB/s of weight.  Bound by the weight stream plus about 7 us of launch, first bytes
 //     and combine, as for the other kinds.
+//   * A gated activation folds neighbouring columns where the finished tile is stored.  Without it here these calls took
+//     the tiled kernel, which cannot cut K for them: 8 x 8192 x 4096 bf16 33.5 us, 22.5 us here.
 //   * The kernel is launched with programmatic stream serialisation: set-up, and for a weight
 //     the caller declares static also the first ring of weight tiles, overlap the tail of the
 //     preceding kernel (the activation quantiser); everything else waits for it.
@@ -39,6 +41,7 @@
 
 #include "gemm.cuh"
 #include "gemm_decode.cuh"
+#include "gemm_epilogue.cuh"
 #include "gemm_tiles.cuh"
 #include "ptx.cuh"
 
@@ -139,11 +142,19 @@ struct UnitWalk {
     }
 };
 
-// out = ((x * s1) * s2) [* row_scale[row]] [* col_scale[col]], the order of the tiled kernels' epilogue
-__device__ __forceinline__ void store_out(const GemmArgs& args, int row, int col, float x, float s1, float s2, float cs) {
+// out = ((x * s1) * s2) [* row_scale[row]] [* col_scale[col]], the order of the tiled kernels' epilogue; a gated activation
+// folds the columns of two neighbouring lanes.  Called by whole warps (a lane is a column; `col_ok`: it is in range).
+__device__ __forceinline__ void store_out(const GemmArgs& args, int row, int col, float x, float s1, float s2, float cs, bool col_ok) {
     x = __fmul_rn(__fmul_rn(x, s1), s2);
     if (args.row_scale != nullptr) x = __fmul_rn(x, args.row_scale[row]);
     if (args.col_scale != nullptr) x = __fmul_rn(x, cs);
+    if (args.act != DSL_ACT_NONE) {
+        const float up = __shfl_down_sync(0xFFFFFFFFu, x, 1);
+        if (col & 1) return;
+        x = glu_value(args.act == DSL_ACT_GEGLU, x, up);
+        col >>= 1;
+    }
+    if (!col_ok) return;
     const size_t off = static_cast<size_t>(row) * args.ldc + col;
     if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off] = __float2bfloat16_rn(x);
     else static_cast<float*>(args.c)[off] = x;
@@ -464,6 +475,30 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                                 if (args.row_scale != nullptr) x[j] = __fmul_rn(x[j], rs);
                                 if (args.col_scale != nullptr) x[j] = __fmul_rn(x[j], cs8[j]);
                             }
+                            if (args.act != DSL_ACT_NONE) {      // (gate, up) pairs: four outputs
+                                float o[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) o[j] = glu_value(args.act == DSL_ACT_GEGLU, x[2 * j], x[2 * j + 1]);
+                                const size_t off = static_cast<size_t>(r) * args.ldc + (colg >> 1);
+                                if (colg + 8 <= args.n && args.ldc % 4 == 0) {
+                                    if (args.out_bf16) {
+                                        const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                                        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(args.c) + off) =
+                                            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                                    } else {
+                                        *reinterpret_cast<float4*>(static_cast<float*>(args.c) + off) = make_float4(o[0], o[1], o[2], o[3]);
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j) {
+                                        if (colg + 2 * j + 1 < args.n) {
+                                            if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + j] = __float2bfloat16_rn(o[j]);
+                                            else static_cast<float*>(args.c)[off + j] = o[j];
+                                        }
+                                    }
+                                }
+                                continue;
+                            }
                             const size_t off = static_cast<size_t>(r) * args.ldc + colg;
                             if (vec && args.out_bf16) {
                                 uint32_t w4[4];
@@ -516,18 +551,17 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const float cs = (col_ok && args.col_scale != nullptr) ? args.col_scale[col] : 1.0f;
             if (KIND == KIND_F8G && whole) {
 #pragma unroll 1
-                for (int row = 0; col_ok && row < args.m_total; ++row) store_out(args, row, col, recv[row * 128 + nl], s1, s2, cs);
+                for (int row = 0; row < args.m_total; ++row) store_out(args, row, col, recv[row * 128 + nl], s1, s2, cs, col_ok);
             } else if (whole) {
 #pragma unroll 1
                 for (int c = 0; c < TOK / 4; ++c) {      // short body: this code runs from a cold instruction cache
                     uint32_t v[4];
                     tmem_ld_32x32b_x4(tmem_base + acc * 128 + c * 4 + lane_base, v);
                     tmem_ld_wait();
-                    if (!col_ok) continue;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int row = c * 4 + i;
-                        if (row < args.m_total) store_out(args, row, col, __uint_as_float(v[i]), s1, s2, cs);
+                        if (row < args.m_total) store_out(args, row, col, __uint_as_float(v[i]), s1, s2, cs, col_ok);
                     }
                 }
                 tc_fence_before();
@@ -581,7 +615,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 if (!epilogue_sync()) { ok = false; break; }
                 if (*last_flag != 0u) {
                     __threadfence();
-                    if (col_ok) {
+                    {
                         // Runs once per launch from a cold instruction cache: kept short.  Four rows in flight
                         // hide part of the L2 latency of the partial tiles.
 #pragma unroll 1
@@ -596,7 +630,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                             }
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
-                                if (row0 + j < args.m_total) store_out(args, row0 + j, col, sum[j], s1, s2, cs);
+                                if (row0 + j < args.m_total) store_out(args, row0 + j, col, sum[j], s1, s2, cs, col_ok);
                         }
                     }
                     if (warp == 2 && lane == 0) *reinterpret_cast<volatile unsigned long long*>(plan.arrivals + tile) = 0ull;
@@ -764,8 +798,7 @@ static bool plan_decode_kind(const GemmArgs& args, size_t* wanted) {
 }
 
 static bool decode_domain(const GemmArgs& args) {
-    return args.group_offsets == nullptr && args.m_total <= DSL_DECODE_MAX_ROWS && args.act == DSL_ACT_NONE &&
-           args.out_sf == nullptr;
+    return args.group_offsets == nullptr && args.m_total <= DSL_DECODE_MAX_ROWS && args.out_sf == nullptr;
 }
 
 size_t decode_scratch_bytes(int kind, const GemmArgs& args, bool* served) {

@@ -11,7 +11,8 @@
 // and scales (98 us, 4.6 TB/s, on the tiled kernel).  A group with more than TOK rows is several items on the same weight tile,
 // neighbours in the order, so that all but the first find it in the L2.
 //
-// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue.  Group-scaled FP8 promotes every K group through registers (promote_run).  Every mbarrier
+// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue.  Group-scaled FP8 promotes every
+// K group through registers (promote_run).  Every mbarrier
 // wait is bounded.
 #include <cuda_bf16.h>
 #include <stdlib.h>
