@@ -257,18 +257,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                 const int col0 = ti.n0 + c * 32;
                 if (!row_ok || col0 >= args.n) continue;
                 if (split_k > 1) {
-                    // raw fp32 partial sums of this K-slice; scales are applied by the reduction
-                    float* dst = args.partial + (static_cast<size_t>(ks) * args.m_total + row) * args.n + col0;
-                    if (args.n % 4 == 0 && col0 + 32 <= args.n) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            reinterpret_cast<float4*>(dst)[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                                                            __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.n) dst[i] = __uint_as_float(v[i]);
-                    }
+                    store_partial32(args, ks, row, col0, true, v);
                 } else {
                     store_chunk32(args, row, col0, ti.group, v, s1, s2, rs, vec_ok, ti.mtile, quad * 32 + lane);
                 }
@@ -335,6 +324,17 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmArgs args,
         x[i] = __fmul_rn(__fmul_rn(acc[i], s1), s2);
         if (args.row_scale != nullptr) x[i] = __fmul_rn(x[i], rs);
         if (args.col_scale != nullptr && col0 + i < args.n) x[i] = __fmul_rn(x[i], args.col_scale[col0 + i]);
+    }
+    if (args.act != DSL_ACT_NONE) {       // (gate, up) pairs: two outputs per thread
+        const bool geglu = args.act == DSL_ACT_GEGLU;
+        const size_t off = static_cast<size_t>(row) * args.ldc + (col0 >> 1);
+        for (int i = 0; i < 2; ++i) {
+            if (col0 + 2 * i + 1 >= args.n) break;
+            const float o = glu_value(geglu, x[2 * i], x[2 * i + 1]);
+            if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + i] = __float2bfloat16_rn(o);
+            else static_cast<float*>(args.c)[off + i] = o;
+        }
+        return;
     }
     const size_t off = static_cast<size_t>(row) * args.ldc + col0;
     if (vec && args.ldc % 4 == 0) {
@@ -459,11 +459,41 @@ static int launch_one(const void* A, const void* B, const GemmArgs& args, long l
     long long grid = items < sm_count() ? items : sm_count();
     if (grid < 1) grid = 1;
     gemm_kernel<KIND, BLOCK_N><<<static_cast<unsigned>(grid), 192, C::SMEM_BYTES, st>>>(ta, tb, args);
-    if (args.split_k > 1) {
-        const long long threads = static_cast<long long>(args.m_total) * ((args.n + 3) / 4);
-        splitk_reduce_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(args, args.split_k);
-    }
+    if (args.split_k > 1) return launch_splitk_reduce(args, st);
     return static_cast<int>(cudaGetLastError());
+}
+
+int launch_splitk_reduce(const GemmArgs& args, cudaStream_t st) {
+    const long long threads = static_cast<long long>(args.m_total) * ((args.n + 3) / 4);
+    splitk_reduce_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(args, args.split_k);
+    return static_cast<int>(cudaGetLastError());
+}
+
+// K slices for a CTA-pair kernel.  A dense problem of few 256 x 256 tiles leaves pairs idle for its whole length (256 x 4096:
+// 16 of 74 busy); cut along K it fills them, at the price of a reduction over the slices' fp32 sums.  Estimated in SM
+// clocks: rounds of the grid x K stages per slice x clocks per stage, plus the reduction (a launch, and the sums written and
+// read once at about 3500 bytes a clock).  Taken when it saves a tenth; the scratch is held to 64 MB.  us per call whole / cut,
+// K = 14336, N = 4096: bf16 200 rows 70.8 / 39.3, 400 rows 71.2 / 54.0; FP8 128x128 blocks 62.9 / 37.8, 62.1 / 51.8; FP8
+// SwiGLU 54.1 / 42.7.  Not where more than half of the pairs have a tile: 1500 rows (96 tiles, two rounds) 146 / 155.
+int choose_pair_split(int kind, const GemmArgs& args) {
+    if (args.group_offsets != nullptr || args.partial == nullptr || args.out_sf != nullptr || args.m_total <= 0 || args.n <= 0) return 1;
+    const int num_kb = (args.k_bytes + STAGE_KB - 1) / STAGE_KB;
+    const long long tiles = ((args.m_total + 255ll) / 256) * ((args.n + 255ll) / 256);
+    const int pairs = sm_count() / 2;
+    if (pairs < 1 || tiles * 2 > pairs || num_kb < 8) return 1;
+    const double stage = kind == KIND_F8G ? 1200 : (kind == KIND_F8 ? 680 : 830);        // measured clocks per 128-byte K stage
+    const double whole = static_cast<double>(num_kb) * stage;
+    const size_t per_slice = static_cast<size_t>(args.m_total) * args.n * sizeof(float);
+    size_t room = args.partial_bytes < (64u << 20) ? args.partial_bytes : (64u << 20);
+    int best = 1;
+    double best_cost = 0.9 * whole;
+    for (int s = 2; s <= 8 && s * 4 <= num_kb && s * per_slice <= room; ++s) {
+        const int per = (num_kb + s - 1) / s;
+        if ((num_kb + per - 1) / per != s) continue;                 // every slice non-empty
+        const double cost = static_cast<double>((tiles * s + pairs - 1) / pairs) * per * stage + 6000 + 2.0 * s * per_slice / 3500;
+        if (cost < best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
 }
 
 // Which kernel serves a problem: the CTA-pair kernel (256x256 tiles) once there is more than
@@ -517,8 +547,11 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args) {
         const size_t b = decode_scratch_bytes(kind, args, &served);
         if (served) return b > 0 ? b + DSL_WS_HEADER_BYTES : 0;
     }
-    if (kind == KIND_F8G) return 0;      // its tiled kernels never split K
-    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) return 0;
+    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) {
+        const int s = choose_pair_split(kind, args);
+        return s > 1 ? DSL_WS_HEADER_BYTES + static_cast<size_t>(s) * args.m_total * args.n * sizeof(float) : 0;
+    }
+    if (kind == KIND_F8G) return 0;      // its 1-CTA kernel never splits K
     long long max_tiles = 0;
     one_cta_tiles(args, &max_tiles);
     const int split_k = choose_split_k(args, max_tiles);
@@ -547,7 +580,10 @@ int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStrea
         if (rc == DSL_NOT_SERVED) rc = launch_gemm_decode_grouped(kind, A, B, args, st);
         if (rc != DSL_NOT_SERVED) return rc;
     }
-    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) return launch_gemm_pair(kind, A, B, args, st);
+    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) {
+        args.split_k = choose_pair_split(kind, args);
+        return launch_gemm_pair(kind, A, B, args, st);
+    }
     long long max_tiles = 0;
     const bool narrow = one_cta_tiles(args, &max_tiles);
     if (args.band <= 0) args.band = 8;

@@ -86,6 +86,8 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args);
 // weight-streaming kernel read it MN-major; the 1-CTA kernels do not).
 bool kn_served(int kind, const GemmArgs& args);
 int choose_split_k(const GemmArgs& args, long long tiles);
+int choose_pair_split(int kind, const GemmArgs& args);
+int launch_splitk_reduce(const GemmArgs& args, cudaStream_t st);
 int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st);
 int launch_gemm_pair(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st);
 int launch_gemm_fp8_groupwise_pair(const void* A, const void* B, GemmArgs args, cudaStream_t st);

@@ -48,6 +48,22 @@ __device__ __forceinline__ float glu_value(bool geglu, float gate, float up) {
     return __fmul_rn(__fdividef(gate, 1.0f + __expf(-z)), up);
 }
 
+// Raw fp32 sums of K slice `ks` (32 columns of a row) to the split-K scratch; the reduction applies scales and activation.
+__device__ __forceinline__ void store_partial32(const GemmArgs& args, int ks, int row, int col0, bool row_ok, const uint32_t (&v)[32]) {
+    if (!row_ok || col0 >= args.n) return;
+    float* dst = args.partial + (static_cast<size_t>(ks) * args.m_total + row) * args.n + col0;
+    if (args.n % 4 == 0 && col0 + 32 <= args.n) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            reinterpret_cast<float4*>(dst)[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                            __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (col0 + i < args.n) dst[i] = __uint_as_float(v[i]);
+    }
+}
+
 // v: 32 fp32 accumulators (bit patterns) of row `row`, columns col0..col0+31 of group `group`.
 // out = (acc * s1) * s2 [* row_scale[row]] [* col_scale[group*n + col]]
 // sf_tile / rin: only read when the result is quantised (args.out_sf != nullptr).

@@ -123,8 +123,8 @@ __device__ __forceinline__ void fma_pair(float& a0, float& a1, uint32_t p0, uint
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
 }
 
-template <bool SB_BLOCK, bool ACT, int PIECES, int RING, bool FMA2 = true>
-__device__ __forceinline__ bool promote_tile(const GemmArgs& args, const gwp::Tile& ti, int num_kb, int nb128, uint32_t tmem_base,
+template <bool SB_BLOCK, bool ACT, bool SPLIT, int PIECES, int RING, bool FMA2 = true>
+__device__ __forceinline__ bool promote_tile(const GemmArgs& args, const gwp::Tile& ti, int num_kb, int ks, int kb0, int kb1, int nb128, uint32_t tmem_base,
                                              uint64_t* part_full, uint64_t* part_empty, volatile uint32_t* abort_flag,
                                              uint32_t& step, int rank, int quad, int half, int lane, int buf_cols) {
     using namespace gwp;
@@ -142,12 +142,12 @@ __device__ __forceinline__ bool promote_tile(const GemmArgs& args, const gwp::Ti
     float acc[PIECES * 16];
 #pragma unroll
     for (int i = 0; i < PIECES * 16; ++i) acc[i] = 0.f;
-    float sa_next = __ldg(sa_row);
-    float sb_next = SB_BLOCK ? __ldg(sb_ptr) : 0.f;
-    for (int kb = 0; kb < num_kb; ++kb, ++step) {
+    float sa_next = __ldg(sa_row + kb0);
+    float sb_next = SB_BLOCK ? __ldg(sb_ptr + kb0) : 0.f;
+    for (int kb = kb0; kb < kb1; ++kb, ++step) {
         const float sa = sa_next;
         const float s = SB_BLOCK ? __fmul_rn(sa, sb_next) : 0.f;
-        if (kb + 1 < num_kb) {   // next group's scales are fetched while this one is promoted
+        if (kb + 1 < kb1) {   // next group's scales are fetched while this one is promoted
             sa_next = __ldg(sa_row + kb + 1);
             if (SB_BLOCK) sb_next = __ldg(sb_ptr + kb + 1);
         }
@@ -202,12 +202,18 @@ __device__ __forceinline__ bool promote_tile(const GemmArgs& args, const gwp::Ti
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(acc[c * 32 + i]);
+        if (SPLIT) {
+            store_partial32(args, ks, row, col0, true, v);
+            continue;
+        }
         store_chunk32_t<ACT>(args, row, col0, ti.group, v, s1, s2, rs, vec_ok);
     }
     return true;
 }
 
-template <bool SB_BLOCK, bool ACT, bool FMA2 = true>
+// SPLIT: the K groups are cut into args.split_k slices (whole tiles only) whose fp32 sums go to scratch.  A variant of its own:
+// the slice bounds cost the promotion loop the registers it has not got (spills).
+template <bool SB_BLOCK, bool ACT, bool FMA2 = true, bool SPLIT = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gwp::THREADS, 1)
 gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                const __grid_constant__ CUtensorMap tmap_b_narrow, const GemmArgs args) {
@@ -283,15 +289,20 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
     tw.plan(num_pairs);
     if (args.whole_tiles_only) { tw.full = tw.total; tw.items = tw.total; }
     const int num_kb = args.k_bytes / STAGE_KB;   // K % 128 == 0
+    // split-K (whole tiles only): work item = tile * split_k + slice; slice ks covers the K groups [ks * kb_per, ...)
+    const int split_k = SPLIT ? args.split_k : 1;
+    const int kb_per = !SPLIT ? num_kb : (num_kb + split_k - 1) / split_k;
+    const int items = tw.items * split_k;
 
     if (warp == 0) {
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int t = pair_id; t < tw.items && ok; t += num_pairs) {
-            const Tile ti = tw.decode(t);
+        for (int t = pair_id; t < items && ok; t += num_pairs) {
+            const Tile ti = tw.decode(t / split_k);
+            const int kb0 = SPLIT ? t % split_k * kb_per : 0, kb1 = SPLIT ? min(num_kb, kb0 + kb_per) : num_kb;
             const bool narrow = ti.width != TILE_N;
-            for (int kb = 0; kb < num_kb; ++kb) {
+            for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait_cluster(empty_bar + stage, phase ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
                 if (elect_one()) {
                     mbar_arrive_expect_tx(full_bar + stage, A_STAGE + (narrow ? B_NARROW : B_STAGE));
@@ -323,12 +334,13 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
             uint32_t phase = 0;
             uint32_t step = 0;   // only its two low bits matter (buffer and phase)
             bool ok = true;
-            for (int t = pair_id; t < tw.items && ok; t += num_pairs) {
+            for (int t = pair_id; t < items && ok; t += num_pairs) {
+                const int kb0 = SPLIT ? t % split_k * kb_per : 0, kb1 = SPLIT ? min(num_kb, kb0 + kb_per) : num_kb;
                 // A narrow piece is always a pair's last item (there are at most as many as pairs).  Its partial products
                 // go through a ring of four 64-column buffers of their own barriers: with the short MMA the round trip
                 // MMA -> promotion -> "buffer free" would otherwise set the pace.  The four buffers lie in the columns
                 // of full-width buffer 0, so its last reader must have finished first.
-                const bool narrow = t >= tw.full;
+                const bool narrow = t / split_k >= tw.full;
                 if (narrow) {
                     const uint32_t next0 = (step + 1u) & ~1u;   // the step that would use buffer 0 next
                     if (!mbar_wait_cluster(part_empty + 0, ((next0 >> 1) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
@@ -340,7 +352,7 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
                 const uint32_t ring = narrow ? NARROW_RING : 2;
                 const uint32_t ring_shift = narrow ? 2 : 1;
                 const uint32_t buf_cols = narrow ? NARROW_N : TILE_N;
-                for (int kb = 0; kb < num_kb; ++kb, ++step) {
+                for (int kb = kb0; kb < kb1; ++kb, ++step) {
                     const uint32_t p = step & (ring - 1u);
                     const uint32_t pphase = (step >> ring_shift) & 1u;
                     if (!mbar_wait_cluster(acc_empty + p, pphase ^ 1u, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
@@ -364,8 +376,9 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int t = pair_id; t < tw.items && ok; t += num_pairs) {
-                for (int kb = 0; kb < num_kb; ++kb) {
+            for (int t = pair_id; t < items && ok; t += num_pairs) {
+                const int kb0 = SPLIT ? t % split_k * kb_per : 0, kb1 = SPLIT ? min(num_kb, kb0 + kb_per) : num_kb;
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(full_bar + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     if (lane == 0) mbar_arrive_cluster(peer_full + stage, 0);
                     __syncwarp();
@@ -380,16 +393,17 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
         const int nb128 = (args.n + 127) / 128;
         uint32_t step = 0;
         bool ok = true;
-        for (int t = pair_id; t < tw.items && ok; t += num_pairs) {
-            const Tile ti = tw.decode(t);
+        for (int t = pair_id; t < items && ok; t += num_pairs) {
+            const Tile ti = tw.decode(t / split_k);
+            const int ks = SPLIT ? t % split_k : 0, kb0 = ks * kb_per, kb1 = SPLIT ? min(num_kb, kb0 + kb_per) : num_kb;
             // full width: TILE_N / PARTS columns per warp, two buffers; a 64-column piece (a pair's last item) goes to the
             // warps of the first two parts, 32 columns each, through its own ring
-            if (ti.width == TILE_N) {
-                ok = promote_tile<SB_BLOCK, ACT, TILE_N / (16 * PARTS), 2, FMA2>(args, ti, num_kb, nb128, tmem_base, part_full, part_empty,
+            if (SPLIT || ti.width == TILE_N) {
+                ok = promote_tile<SB_BLOCK, ACT, SPLIT, TILE_N / (16 * PARTS), 2, FMA2>(args, ti, num_kb, ks, kb0, kb1, nb128, tmem_base, part_full, part_empty,
                                                                                  abort_flag, step, static_cast<int>(rank), quad, part, lane, TILE_N);
-            } else if (part < 2) {
+            } else if (!SPLIT && part < 2) {
                 uint32_t nstep = 0;
-                ok = promote_tile<SB_BLOCK, ACT, NARROW_N / 32, NARROW_RING, FMA2>(args, ti, num_kb, nb128, tmem_base, nar_full, nar_empty,
+                ok = promote_tile<SB_BLOCK, ACT, SPLIT, NARROW_N / 32, NARROW_RING, FMA2>(args, ti, num_kb, ks, kb0, kb1, nb128, tmem_base, nar_full, nar_empty,
                                                                              abort_flag, nstep, static_cast<int>(rank), quad, part, lane, NARROW_N);
             }
         }
@@ -411,7 +425,7 @@ gemm_fp8_groupwise_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const
     }
 }
 
-template <bool SB_BLOCK, bool ACT, bool FMA2 = true>
+template <bool SB_BLOCK, bool ACT, bool FMA2 = true, bool SPLIT = false>
 static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cudaStream_t st) {
     CUtensorMap ta, tb, tbn;
     const int groups = args.group_offsets != nullptr ? args.num_groups : 1;
@@ -428,7 +442,7 @@ static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cu
     if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
     int max_clusters = clusters_of.v[dev].load(std::memory_order_acquire);
     if (max_clusters == 0) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2, SPLIT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, gwp::SMEM_BYTES);
         if (e != cudaSuccess) return static_cast<int>(e);
         const int sms = sm_count();
@@ -437,7 +451,7 @@ static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cu
         cfg.blockDim = dim3(gwp::THREADS);
         cfg.dynamicSmemBytes = gwp::SMEM_BYTES;
         int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2>, &cfg);
+        e = cudaOccupancyMaxActiveClusters(&n, gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2, SPLIT>, &cfg);
         max_clusters = (e == cudaSuccess && n > 0) ? n : (sms > 1 ? sms / 2 : 1);
         (void)cudaGetLastError();
         clusters_of.v[dev].store(max_clusters, std::memory_order_release);
@@ -445,7 +459,8 @@ static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cu
     const long long m_tiles_max = (args.m_total + gwp::TILE_M - 1) / gwp::TILE_M + groups - 1;
     const long long max_tiles = m_tiles_max * ((args.n + gwp::TILE_N - 1) / gwp::TILE_N);
     if (max_tiles > (1ll << 29)) return DSL_ERR_SHAPE;   // tile counters in the kernel are 32-bit
-    long long clusters = max_tiles < max_clusters ? max_tiles : max_clusters;
+    const long long max_items = max_tiles * (SPLIT ? args.split_k : 1);      // split only for few tiles
+    long long clusters = max_items < max_clusters ? max_items : max_clusters;
     if (clusters < 1) clusters = 1;
     // Launched with programmatic stream serialisation: the grid's set-up overlaps the tail of the preceding kernel
     // of the stream when that kernel allows it (the quantisers do); the kernel's griddep_wait() guards the rest.
@@ -461,7 +476,9 @@ static int launch_gw_pair(const void* A, const void* B, const GemmArgs& args, cu
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2>, ta, tb, tbn, args));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_groupwise_pair_kernel<SB_BLOCK, ACT, FMA2, SPLIT>, ta, tb, tbn, args);
+    if (e != cudaSuccess || !SPLIT) return static_cast<int>(e);
+    return launch_splitk_reduce(args, st);
 }
 
 // The kernel's work list, computed on the host with the kernel's own Walker (no CUDA call): item i of the launch goes
@@ -509,8 +526,11 @@ int launch_gemm_fp8_groupwise_pair(const void* A, const void* B, GemmArgs args, 
     if (args.band <= 0) args.band = 8;
     {   // DSLGEMM_WHOLE_TILES=1 keeps every tile whole (for measurements)
         static const int whole = [] { const char* e = getenv("DSLGEMM_WHOLE_TILES"); return (e != nullptr && e[0] == '1') ? 1 : 0; }();
-        args.whole_tiles_only = whole || args.b_kn;      // a 32-column half of a piece is no whole 128-byte block of an MN-major tile
+        args.split_k = choose_pair_split(KIND_F8G, args);
+        args.whole_tiles_only = whole || args.b_kn || args.split_k > 1;      // a 32-column half of a piece is no whole 128-byte block of an MN-major tile
     }
+    if (args.split_k > 1)      // the reduction over the slices applies the activation too
+        return args.sb_block ? launch_gw_pair<true, false, true, true>(A, B, args, st) : launch_gw_pair<false, false, true, true>(A, B, args, st);
     // two instantiations: the plain epilogue keeps the promotion loop free of spills, the activation one is larger
     if (args.act != DSL_ACT_NONE)
         return args.sb_block ? launch_gw_pair<true, true>(A, B, args, st) : launch_gw_pair<false, true>(A, B, args, st);

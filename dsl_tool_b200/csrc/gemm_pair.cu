@@ -179,17 +179,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tw.total = static_cast<long long>(tw.m_tiles) * tw.n_tiles;
     const int num_kb = (args.k_bytes + STAGE_KB - 1) / STAGE_KB;
     const int sf_tiles_total = s_sft0[groups];
+    // split-K: work item = tile * split_k + slice; slice ks covers the K stages [ks * kb_per, ...) and leaves fp32 sums
+    const int split_k = args.split_k > 1 ? args.split_k : 1;
+    const int kb_per = (num_kb + split_k - 1) / split_k;
+    const long long total_items = tw.total * split_k;
 
     if (warp == 0) {
         // ================= TMA producer (each CTA loads its own halves) =================
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (long long t = pair_id; t < tw.total && ok; t += num_pairs) {
-            const pr::PairTile ti = tw.decode(t);
+        for (long long t = pair_id; t < total_items && ok; t += num_pairs) {
+            const pr::PairTile ti = tw.decode(t / split_k);
+            const int kb0 = static_cast<int>(t % split_k) * kb_per;
+            const int kb1 = min(num_kb, kb0 + kb_per);
             const int my_sf_tile = ti.sf_tile + static_cast<int>(rank);
             const bool sfa_valid = C::SF_ATOMS > 0 && my_sf_tile < sf_tiles_total;
-            for (int kb = 0; kb < num_kb; ++kb) {
+            for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait_cluster(empty_bar + stage, phase ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
                 if (elect_one()) {
                     uint32_t bytes = C::A_STAGE + C::B_STAGE;
@@ -251,7 +257,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             uint32_t phase = 0;
             bool ok = true;
             long long iter = 0;
-            for (long long t = pair_id; t < tw.total && ok; t += num_pairs, ++iter) {
+            for (long long t = pair_id; t < total_items && ok; t += num_pairs, ++iter) {
+                const int kb0 = static_cast<int>(t % split_k) * kb_per;
+                const int kb1 = min(num_kb, kb0 + kb_per);
                 const int acc = static_cast<int>(iter % C::ACC_STAGES);
                 const uint32_t acc_phase = static_cast<uint32_t>((iter / C::ACC_STAGES) & 1);
                 if (!mbar_wait_cluster(acc_empty + acc, acc_phase ^ 1u, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
@@ -259,7 +267,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     !mbar_wait_cluster(ovl_free, static_cast<uint32_t>((iter - 1) & 1), abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * C::ACC1_COL;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(full_bar + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     if (!mbar_wait_cluster(peer_full + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     tc_fence_after();
@@ -282,7 +290,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                         }
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
+                            const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
                             if (KIND == KIND_F8) {
                                 mma_f8f6f4_pair(d_tmem, adesc + 2 * k, bdesc + b_step * k, idesc, accum);
                             } else if (KIND == KIND_BF16) {
@@ -298,7 +306,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                             }
                         }
                         tc_commit_pair(empty_bar + stage);
-                        if (kb == num_kb - 1) tc_commit_pair(acc_full + acc);
+                        if (kb == kb1 - 1) tc_commit_pair(acc_full + acc);
                     }
                     __syncwarp();
                     if (++stage == C::NUM_STAGES) { stage = 0; phase ^= 1u; }
@@ -309,8 +317,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (long long t = pair_id; t < tw.total && ok; t += num_pairs) {
-                for (int kb = 0; kb < num_kb; ++kb) {
+            for (long long t = pair_id; t < total_items && ok; t += num_pairs) {
+                const int kb0 = static_cast<int>(t % split_k) * kb_per;
+                const int kb1 = min(num_kb, kb0 + kb_per);
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(full_bar + stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     if (lane == 0) mbar_arrive_cluster(peer_full + stage, 0);
                     __syncwarp();
@@ -326,12 +336,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (args.scale_product) { s1 = s1 * s2; s2 = 1.0f; }
         const bool vec_ok = args.out_bf16 ? (args.ldc % 8 == 0) : (args.ldc % 4 == 0);
         // plain bf16 results leave through the warp-wide store (rows exchanged in shared memory)
-        const bool warp_store = args.out_bf16 && vec_ok && args.act == DSL_ACT_NONE && args.out_sf == nullptr;
+        const bool warp_store = split_k == 1 && args.out_bf16 && vec_ok && args.act == DSL_ACT_NONE && args.out_sf == nullptr;
         uint8_t* epi_scratch = smem + C::OFF_EPI + (warp - 2) * 2048;
         bool ok = true;
         long long iter = 0;
-        for (long long t = pair_id; t < tw.total && ok; t += num_pairs, ++iter) {
-            const pr::PairTile ti = tw.decode(t);
+        for (long long t = pair_id; t < total_items && ok; t += num_pairs, ++iter) {
+            const pr::PairTile ti = tw.decode(t / split_k);
+            const int ks = static_cast<int>(t % split_k);
             const int acc = static_cast<int>(iter % C::ACC_STAGES);
             const uint32_t acc_phase = static_cast<uint32_t>((iter / C::ACC_STAGES) & 1);
             if (!mbar_wait_cluster(acc_full + acc, acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
@@ -363,12 +374,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 }
                 if (warp_store && ti.n0 + ca * 32 + 32 <= args.n)
                     store_chunk32_bf16_warp(args, epi_scratch, row_warp, ti.row_end, ti.n0 + ca * 32, ti.group, va, s1, s2, rs, lane);
+                else if (split_k > 1)
+                    store_partial32(args, ks, row, ti.n0 + ca * 32, row_ok, va);
                 else if (row_ok && ti.n0 + ca * 32 < args.n)
                     store_chunk32(args, row, ti.n0 + ca * 32, ti.group, va, s1, s2, rs, vec_ok, ti.sf_tile + static_cast<int>(rank), quad * 32 + lane);
                 tmem_ld_wait();
                 if (j + 2 < pr::TILE_N / 32) tmem_ld_32x32b_x32(t_row + (rot ? ((j + 8) & 7) : j + 2) * 32, va);
                 if (warp_store && ti.n0 + cb * 32 + 32 <= args.n)
                     store_chunk32_bf16_warp(args, epi_scratch, row_warp, ti.row_end, ti.n0 + cb * 32, ti.group, vb, s1, s2, rs, lane);
+                else if (split_k > 1)
+                    store_partial32(args, ks, row, ti.n0 + cb * 32, row_ok, vb);
                 else if (row_ok && ti.n0 + cb * 32 < args.n)
                     store_chunk32(args, row, ti.n0 + cb * 32, ti.group, vb, s1, s2, rs, vec_ok, ti.sf_tile + static_cast<int>(rank), quad * 32 + lane);
             }
@@ -426,7 +441,8 @@ static int launch_pair_one(const void* A, const void* B, const GemmArgs& args, l
         if (getenv("DSLGEMM_DEBUG") != nullptr) fprintf(stderr, "[dslgemm] pair kernel kind %d: %d resident clusters (occupancy query %s)\n", KIND, max_clusters, cudaGetErrorName(e));
         clusters_of.v[dev].store(max_clusters, std::memory_order_release);
     }
-    long long clusters = max_tiles < max_clusters ? max_tiles : max_clusters;
+    const long long max_items = max_tiles * (args.split_k > 1 ? args.split_k : 1);
+    long long clusters = max_items < max_clusters ? max_items : max_clusters;
     if (clusters < 1) clusters = 1;
     // Launched with programmatic stream serialisation: the grid's set-up (barriers, tensor-memory allocation)
     // overlaps the tail of the preceding kernel of the stream when that kernel allows it (the quantisers do);
@@ -442,7 +458,9 @@ static int launch_pair_one(const void* A, const void* B, const GemmArgs& args, l
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<KIND>, ta, tb, args));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<KIND>, ta, tb, args);
+    if (e != cudaSuccess || args.split_k <= 1) return static_cast<int>(e);
+    return launch_splitk_reduce(args, st);
 }
 
 int launch_gemm_pair(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st) {
