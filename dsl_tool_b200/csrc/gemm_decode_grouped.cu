@@ -122,7 +122,9 @@ gemm_decode_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
         fence_proxy_async_smem();
     }
     if (warp == 1) tmem_alloc(tmem_ptr, TMEM_COLS);
-    // Everything above touches no global memory and may overlap the tail of the preceding kernel of the stream.
+    // Everything above touches no global memory and may overlap the tail of the preceding kernel of the stream; a successor
+    // that opted in may be placed on an SM as soon as this kernel's CTA leaves it.
+    griddep_launch_dependents();
     griddep_wait();
     load_group_offsets(s_offs, args.group_offsets, groups, args.m_total);
     __syncthreads();

@@ -117,8 +117,12 @@ extern "C" int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int
     const int R = tokens * k;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define DSL_STEP(call) do { rc = (call); if (rc != 0) return rc; } while (0)
-    DSL_STEP(dsl_moe_route(logits, logits_dtype, tokens, E, k, renorm, i32(l.ids), f32(l.weights), stream));
-    DSL_STEP(dsl_moe_plan(i32(l.ids), R, E, i32(l.counts), i32(l.offsets), i32(l.tile0), i32(l.dest), stream));
+    // Routing and plan go out after the quantiser where there is one: they are launched as programmatic dependents (moe.cu),
+    // the quantiser, a kernel of other chains too, is not.
+    auto route_and_plan = [&]() -> int {
+        const int r = dsl_moe_route(logits, logits_dtype, tokens, E, k, renorm, i32(l.ids), f32(l.weights), stream);
+        return r != 0 ? r : dsl_moe_plan(i32(l.ids), R, E, i32(l.counts), i32(l.offsets), i32(l.tile0), i32(l.dest), stream);
+    };
     const int* offs = i32(l.offsets);
     dsl_epilogue up{}, dn{};
     up.scale_a_host = up.scale_b_host = dn.scale_a_host = dn.scale_b_host = 1.0f;
@@ -134,6 +138,7 @@ extern "C" int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int
         float* gs = act_gs_dev != nullptr ? const_cast<float*>(act_gs_dev) : f32(l.gs);
         DSL_STEP(dsl_quant_fp4(x, x_dtype, tokens, K, fmt, fmt == DSL_FP4_NV ? gs : nullptr, act_gs_dev != nullptr, u8(l.q), u8(l.sf),
                                nullptr, 0, u8(l.ws), stream));
+        DSL_STEP(route_and_plan());
         // Scale bytes of rows no group owns only reach result rows that nobody stores; those past the last K block meet
         // zero-filled elements, where a NaN pattern would spread, so they alone have to be cleared.
         if ((K / blk) % 4 != 0) DSL_STEP(static_cast<int>(cudaMemsetAsync(u8(l.row_sf), 0, l.row_sf_bytes, st)));
@@ -163,6 +168,7 @@ extern "C" int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int
                               stream));
     } else if (format == DSL_W_FP8) {
         DSL_STEP(dsl_quant_fp8(x, x_dtype, tokens, K, DSL_FP8_PER_TENSOR, f32(l.gs), 0, u8(l.q), u8(l.ws), stream));
+        DSL_STEP(route_and_plan());
         DSL_STEP(dsl_moe_dispatch_rows(u8(l.q), i32(l.ids), i32(l.dest), i32(l.offsets), tokens, k, K, 0, E, u8(l.rows), stream));
         up.scale_a_dev = f32(l.gs);
         up.scale_b_dev = static_cast<const float*>(gate_up->scale);
@@ -173,6 +179,7 @@ extern "C" int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int
         DSL_STEP(dsl_gemm_fp8(u8(l.hq), wd, y, D, R, D, H, offs, E, &dn, status, stream));
     } else if (format == DSL_W_FP8_BLOCK128) {
         DSL_STEP(dsl_quant_fp8(x, x_dtype, tokens, K, DSL_FP8_GROUP_1X128, f32(l.sf), 0, u8(l.q), u8(l.ws), stream));
+        DSL_STEP(route_and_plan());
         DSL_STEP(dsl_moe_dispatch_rows(u8(l.q), i32(l.ids), i32(l.dest), i32(l.offsets), tokens, k, K, 0, E, u8(l.rows), stream));
         DSL_STEP(dsl_moe_dispatch_rows(u8(l.sf), i32(l.ids), i32(l.dest), i32(l.offsets), tokens, k, K / 128 * 4ll, 0, E, u8(l.row_sf), stream));
         DSL_STEP(dsl_gemm_fp8_groupwise(u8(l.rows), wu, f32(l.row_sf), static_cast<const float*>(gate_up->scale), 1, u8(l.h), H, R,
@@ -181,6 +188,7 @@ extern "C" int dsl_moe_layer(const void* x, int x_dtype, const void* logits, int
         DSL_STEP(dsl_gemm_fp8_groupwise(u8(l.hq), wd, f32(l.h_sf), static_cast<const float*>(down->scale), 1, y, D, R, D, H, offs, E, &dn,
                                         status, stream));
     } else {
+        DSL_STEP(route_and_plan());
         DSL_STEP(dsl_moe_dispatch_rows(x, i32(l.ids), i32(l.dest), i32(l.offsets), tokens, k, 2ll * K, 0, E, u8(l.rows), stream));
         DSL_STEP(dsl_gemm_bf16(u8(l.rows), wu, u8(l.h), H, R, gate_up->n, K, offs, E, &up, status, stream));
         DSL_STEP(dsl_gemm_bf16(u8(l.h), wd, y, D, R, D, H, offs, E, &dn, status, stream));
