@@ -48,6 +48,20 @@ __device__ __forceinline__ float glu_value(bool geglu, float gate, float up) {
     return __fmul_rn(__fdividef(gate, 1.0f + __expf(-z)), up);
 }
 
+// f = (v * s1) * s2 [* rs]; the block-scaled kinds fold both scales into s1, so their second factor is 1 and is left out.
+__device__ __forceinline__ void scale32(const GemmArgs& args, const uint32_t (&v)[32], float s1, float s2, float rs, float (&f)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) f[i] = __fmul_rn(__uint_as_float(v[i]), s1);
+    if (s2 != 1.0f) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = __fmul_rn(f[i], s2);
+    }
+    if (args.row_scale != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = __fmul_rn(f[i], rs);
+    }
+}
+
 // Raw fp32 sums of K slice `ks` (32 columns of a row) to the split-K scratch; the reduction applies scales and activation.
 __device__ __forceinline__ void store_partial32(const GemmArgs& args, int ks, int row, int col0, bool row_ok, const uint32_t (&v)[32]) {
     if (!row_ok || col0 >= args.n) return;
@@ -75,12 +89,7 @@ __device__ __forceinline__ void store_chunk32_t(const GemmArgs& args, int row, i
                                                 const uint32_t (&v)[32], float s1, float s2, float rs, bool vec_ok,
                                                 int sf_tile = 0, int rin = 0) {
     float f[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        float x = __fmul_rn(__fmul_rn(__uint_as_float(v[i]), s1), s2);
-        if (args.row_scale != nullptr) x = __fmul_rn(x, rs);
-        f[i] = x;
-    }
+    scale32(args, v, s1, s2, rs, f);
     if (args.col_scale != nullptr) {
         const float* cs = args.col_scale + static_cast<size_t>(group) * args.n;
 #pragma unroll
@@ -180,12 +189,7 @@ __device__ __forceinline__ void store_chunk32_bf16_warp(const GemmArgs& args, ui
                                                         int col0, int group, const uint32_t (&v)[32], float s1, float s2,
                                                         float rs, int lane) {
     float f[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        float x = __fmul_rn(__fmul_rn(__uint_as_float(v[i]), s1), s2);
-        if (args.row_scale != nullptr) x = __fmul_rn(x, rs);
-        f[i] = x;
-    }
+    scale32(args, v, s1, s2, rs, f);
     if (args.col_scale != nullptr) {
         const float* cs = args.col_scale + static_cast<size_t>(group) * args.n;
 #pragma unroll

@@ -362,16 +362,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const bool rot = C::SF_ATOMS > 0 && acc == 0;
             uint32_t va[32], vb[32];
             tmem_ld_32x32b_x32(t_row + (rot ? 6 : 0) * 32, va);
+            // block-scaled kinds: the next tile's MMAs wait for the two shared chunks, so both loads go out together
+            if (C::SF_ATOMS > 0) tmem_ld_32x32b_x32(t_row + (rot ? 7 : 1) * 32, vb);
 #pragma unroll 1
             for (int j = 0; j < pr::TILE_N / 32; j += 2) {
                 const int ca = rot ? ((j + 6) & 7) : j;
                 const int cb = rot ? ((j + 7) & 7) : j + 1;
                 tmem_ld_wait();
-                tmem_ld_32x32b_x32(t_row + cb * 32, vb);
+                if (C::SF_ATOMS == 0 || j > 0) tmem_ld_32x32b_x32(t_row + cb * 32, vb);
                 if (C::SF_ATOMS > 0 && j == 0) {
                     // chunks 0 and 1 of this walk are the columns shared with the other accumulator: hand them back as
                     // soon as both are in registers, before any of the slower scale / convert / store work
-                    tmem_ld_wait();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(ovl_free, 0);
