@@ -224,7 +224,8 @@ def workspace(device: torch.device, need: int = WORKSPACE_BYTES) -> Optional[tor
             return torch.empty(int(need), dtype=torch.uint8, device=device)
         if t is not None:
             _retired_workspaces.append(t)      # a captured CUDA graph may still point at it
-        t = torch.empty(max(int(need), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
+        # powers of two, so that what a stream has outgrown adds up to less than what it has
+        t = torch.empty(max(1 << (int(need) - 1).bit_length(), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
         _workspace[key] = t
     return t
 

@@ -130,3 +130,47 @@ def test_new_argument_validation_without_gpu(cdll):
     assert cdll.dsl_moe_reduce_pull(ptrs, 2, 0, 0, 64, 1, p, 1, None) == 0                             # nothing to do
     assert cdll.dsl_quant_fp4_ref32(None, 0, 64, p, p, None) == -1
     assert cdll.dsl_gemm_fp4_ref32(p, p, p, p, p, 4, 8, 48, None) == -2                                # K % 32
+
+
+def test_pack_kn_layer_and_kn_operand_validation_without_gpu(cdll):
+    buf = ctypes.create_string_buffer(4096)
+    p = (ctypes.addressof(buf) + 255) & ~255
+    def pack(w=p, dtype=1, G=1, K=64, N=64, fmt=_lib.W_NVFP4, inter=0, scale=p, given=0, q=p, sf=p, nbytes=1 << 20, ws=p):
+        return cdll.dsl_pack_kn(w, dtype, G, K, N, fmt, inter, scale, given, q, sf, nbytes, ws, None)
+    assert pack(w=None) == -1 and pack(scale=None) == -1 and pack(ws=None) == -1 and pack(sf=None) == -1
+    assert pack(dtype=3) == -4 and pack(fmt=9) == -4
+    assert pack(K=48) == -2 and pack(N=60) == -2 and pack(inter=1, N=24) == -2 and pack(inter=1, N=63) == -2 and pack(G=-1) == -2
+    assert pack(dtype=0, N=62) == -2 and pack(fmt=_lib.W_FP8, K=24) == -2 and pack(fmt=_lib.W_BF16, K=12) == -2
+    assert pack(w=p + 8) == -3 and pack(q=p + 8) == -3 and pack(sf=p + 8) == -3
+    assert pack(nbytes=511) == -6 and pack(G=70000) == -6
+    assert pack(G=0) == 0 and pack(K=0) == 0 and pack(N=0) == 0                                            # nothing to do
+    ep = _lib.Epilogue()
+    ep.b_is_kn = 1
+    assert cdll.dsl_gemm_fp4(p, p, p, p, 0, p, 256, 200, 256, 64, None, 1, ctypes.byref(ep), None, None) == -4    # pairs run along K
+    assert cdll.dsl_gemm_fp8(p, p, p, 264, 200, 264, 64, None, 1, ctypes.byref(ep), None, None) == -2              # row pitch
+    assert cdll.dsl_gemm_kn_served(_lib.OP_GEMM_FP8, 200, 272, 64, 1) == 1
+    assert cdll.dsl_gemm_kn_served(_lib.OP_GEMM_FP8, 200, 264, 64, 1) == 0
+    assert cdll.dsl_gemm_kn_served(_lib.OP_GEMM_BF16, 200, 264, 64, 1) == 1
+    assert cdll.dsl_gemm_kn_served(_lib.OP_GEMM_FP4_NV, 200, 272, 64, 1) == 0
+    gu, dn = _lib.Weight(), _lib.Weight()
+    gu.format = dn.format = _lib.W_NVFP4
+    gu.groups = dn.groups = 4
+    gu.n, gu.k, dn.n, dn.k = 128, 64, 96, 64
+    def need(k=2, tokens=8):
+        return cdll.dsl_moe_layer_scratch_bytes(ctypes.byref(gu), ctypes.byref(dn), tokens, k, 0)
+    assert need() > 0 and need(k=5) == 0 and need(k=0) == 0 and need(tokens=-1) == 0
+    dn.k = 32
+    assert need() == 0                                                                                      # hidden sizes differ
+    dn.k, dn.groups = 64, 3
+    assert need() == 0
+    dn.groups, dn.format = 4, _lib.W_MXFP4
+    assert need() == 0
+    dn.format = gu.format = _lib.W_FP8_BLOCK128
+    assert need() == 0                                                                                      # K % 512
+    gu.n, gu.k, dn.k = 256, 512, 128
+    size = need()
+    def layer(scratch=p, nbytes=size, x=p, x_dtype=1):
+        return cdll.dsl_moe_layer(x, x_dtype, p, 0, 8, 2, 1, ctypes.byref(gu), ctypes.byref(dn), None, 0, 1.0, scratch, nbytes, p, 1, None, None)
+    assert size > 0 and layer(x=None) == -1
+    gu.q = dn.q = gu.scale = dn.scale = p
+    assert layer(scratch=p + 16) == -3 and layer(nbytes=size - 1) == -6 and layer(x_dtype=3) == -4
