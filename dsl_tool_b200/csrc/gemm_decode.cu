@@ -172,6 +172,8 @@ __device__ __forceinline__ void bulk_send_to_cta(void* dst_local_equiv, const vo
                  : "memory");
 }
 
+template <bool V> struct BoolConst { static constexpr bool value = V; };
+
 template <int KIND, int TOK>
 __global__ void __launch_bounds__(192, 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -457,71 +459,76 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                         for (int j = 0; j < 8; ++j)
                             cs8[j] = (args.col_scale != nullptr && colg + j < args.n) ? args.col_scale[colg + j] : 1.0f;
                         const bool vec = colg + 8 <= args.n && (args.out_bf16 ? args.ldc % 8 == 0 : args.ldc % 4 == 0);
+                        // two loops, so that the plain one stays as short as it can be (cold instruction cache)
+                        auto finish_rows = [&](auto gated) {
 #pragma unroll 1
-                        for (int r = et >> 4; r < args.m_total; r += 8) {
-                            const float4* src = reinterpret_cast<const float4*>(recv + r * 128 + g8);
-                            float4 a = src[0], b = src[1];
+                            for (int r = et >> 4; r < args.m_total; r += 8) {
+                                const float4* src = reinterpret_cast<const float4*>(recv + r * 128 + g8);
+                                float4 a = src[0], b = src[1];
 #pragma unroll 1
-                            for (int p = 1; p < runs; ++p) {                   // ascending K
-                                const float4 pa = src[p * (TOK * 32)], pb = src[p * (TOK * 32) + 1];
-                                a.x += pa.x; a.y += pa.y; a.z += pa.z; a.w += pa.w;
-                                b.x += pb.x; b.y += pb.y; b.z += pb.z; b.w += pb.w;
-                            }
-                            float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                            const float rs = args.row_scale != nullptr ? args.row_scale[r] : 1.0f;
+                                for (int p = 1; p < runs; ++p) {                   // ascending K
+                                    const float4 pa = src[p * (TOK * 32)], pb = src[p * (TOK * 32) + 1];
+                                    a.x += pa.x; a.y += pa.y; a.z += pa.z; a.w += pa.w;
+                                    b.x += pb.x; b.y += pb.y; b.z += pb.z; b.w += pb.w;
+                                }
+                                float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                                const float rs = args.row_scale != nullptr ? args.row_scale[r] : 1.0f;
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                x[j] = __fmul_rn(__fmul_rn(x[j], s1), s2);
-                                if (args.row_scale != nullptr) x[j] = __fmul_rn(x[j], rs);
-                                if (args.col_scale != nullptr) x[j] = __fmul_rn(x[j], cs8[j]);
-                            }
-                            if (args.act != DSL_ACT_NONE) {      // (gate, up) pairs: four outputs
-                                float o[4];
+                                for (int j = 0; j < 8; ++j) {
+                                    x[j] = __fmul_rn(__fmul_rn(x[j], s1), s2);
+                                    if (args.row_scale != nullptr) x[j] = __fmul_rn(x[j], rs);
+                                    if (args.col_scale != nullptr) x[j] = __fmul_rn(x[j], cs8[j]);
+                                }
+                                if constexpr (decltype(gated)::value) {      // (gate, up) pairs: four outputs
+                                    float o[4];
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) o[j] = glu_value(args.act == DSL_ACT_GEGLU, x[2 * j], x[2 * j + 1]);
-                                const size_t off = static_cast<size_t>(r) * args.ldc + (colg >> 1);
-                                if (colg + 8 <= args.n && args.ldc % 4 == 0) {
-                                    if (args.out_bf16) {
-                                        const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
-                                        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(args.c) + off) =
-                                            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                                    for (int j = 0; j < 4; ++j) o[j] = glu_value(args.act == DSL_ACT_GEGLU, x[2 * j], x[2 * j + 1]);
+                                    const size_t off = static_cast<size_t>(r) * args.ldc + (colg >> 1);
+                                    if (colg + 8 <= args.n && args.ldc % 4 == 0) {
+                                        if (args.out_bf16) {
+                                            const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                                            *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(args.c) + off) =
+                                                make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                                        } else {
+                                            *reinterpret_cast<float4*>(static_cast<float*>(args.c) + off) = make_float4(o[0], o[1], o[2], o[3]);
+                                        }
                                     } else {
-                                        *reinterpret_cast<float4*>(static_cast<float*>(args.c) + off) = make_float4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+                                        for (int j = 0; j < 4; ++j) {
+                                            if (colg + 2 * j + 1 < args.n) {
+                                                if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + j] = __float2bfloat16_rn(o[j]);
+                                                else static_cast<float*>(args.c)[off + j] = o[j];
+                                            }
+                                        }
                                     }
                                 } else {
+                                    const size_t off = static_cast<size_t>(r) * args.ldc + colg;
+                                    if (vec && args.out_bf16) {
+                                        uint32_t w4[4];
 #pragma unroll
-                                    for (int j = 0; j < 4; ++j) {
-                                        if (colg + 2 * j + 1 < args.n) {
-                                            if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + j] = __float2bfloat16_rn(o[j]);
-                                            else static_cast<float*>(args.c)[off + j] = o[j];
+                                        for (int j = 0; j < 4; ++j) {
+                                            __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+                                            w4[j] = *reinterpret_cast<uint32_t*>(&h);
+                                        }
+                                        *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(args.c) + off) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                                    } else if (vec) {
+                                        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(args.c) + off);
+                                        dst[0] = make_float4(x[0], x[1], x[2], x[3]);
+                                        dst[1] = make_float4(x[4], x[5], x[6], x[7]);
+                                    } else {
+#pragma unroll
+                                        for (int j = 0; j < 8; ++j) {
+                                            if (colg + j < args.n) {
+                                                if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + j] = __float2bfloat16_rn(x[j]);
+                                                else static_cast<float*>(args.c)[off + j] = x[j];
+                                            }
                                         }
                                     }
                                 }
-                                continue;
                             }
-                            const size_t off = static_cast<size_t>(r) * args.ldc + colg;
-                            if (vec && args.out_bf16) {
-                                uint32_t w4[4];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-                                    w4[j] = *reinterpret_cast<uint32_t*>(&h);
-                                }
-                                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(args.c) + off) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                            } else if (vec) {
-                                float4* dst = reinterpret_cast<float4*>(static_cast<float*>(args.c) + off);
-                                dst[0] = make_float4(x[0], x[1], x[2], x[3]);
-                                dst[1] = make_float4(x[4], x[5], x[6], x[7]);
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    if (colg + j < args.n) {
-                                        if (args.out_bf16) static_cast<__nv_bfloat16*>(args.c)[off + j] = __float2bfloat16_rn(x[j]);
-                                        else static_cast<float*>(args.c)[off + j] = x[j];
-                                    }
-                                }
-                            }
-                        }
+                        };
+                        if (args.act != DSL_ACT_NONE) finish_rows(BoolConst<true>());
+                        else finish_rows(BoolConst<false>());
                     }
                 }
             }
