@@ -122,10 +122,11 @@ gemm_decode_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
         fence_proxy_async_smem();
     }
     if (warp == 1) tmem_alloc(tmem_ptr, TMEM_COLS);
-    // Everything above touches no global memory and may overlap the tail of the preceding kernel of the stream; a successor
-    // that opted in may be placed on an SM as soon as this kernel's CTA leaves it.
-    griddep_launch_dependents();
+    // Everything above touches no global memory and may overlap the tail of the preceding kernel of the stream.  A successor
+    // that opted in may be placed on an SM as soon as this kernel's CTA leaves it; it is let go only after the wait, because it
+    // may fetch a weight that was complete before this kernel started (dsl_epilogue.b_is_static).
     griddep_wait();
+    griddep_launch_dependents();
     load_group_offsets(s_offs, args.group_offsets, groups, args.m_total);
     __syncthreads();
     if (warp == 2) {   // tables, 32 groups at a time: running maximum (monotone offsets), then running sums of the blocks

@@ -19,11 +19,12 @@ namespace dsl {
 
 // The steps run back to back and each is a few microseconds long, as long as the gap between two launches.  They are launched
 // with programmatic stream serialisation: a step's CTAs are placed while the step before it still runs and wait here, before
-// they touch any memory, until it has completed.  Layer of 64 experts, top 8, NVFP4: 64 tokens 164.5 -> 147 us, one token
-// 70 -> 66 us (launched the plain way / so).
+// they touch any memory, until it has completed.  A step lets its own successor start only after that wait, so that when a
+// kernel of the chain starts, everything before its predecessor is complete: a successor that fetches a weight early
+// (dsl_epilogue.b_is_static) relies on it.
 __device__ __forceinline__ void chain_link() {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
 }
 
 // ---- router: softmax over the experts, top-k ------------------------------------------------

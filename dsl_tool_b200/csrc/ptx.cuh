@@ -238,7 +238,8 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 // Programmatic dependent launch: `griddep_wait` blocks until the kernel that precedes this one in the
 // stream has completed and its writes are visible (no-op for a normally launched kernel);
-// `griddep_launch_dependents` lets a successor that opted in start before this kernel ends.
+// `griddep_launch_dependents` lets a successor that opted in start before this kernel ends.  A kernel that is itself launched
+// as a dependent calls it after `griddep_wait`, else the successor could start while the kernel before this one still runs.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // One lane of a converged warp; keeps the operands of the tcgen05 / TMA instructions that

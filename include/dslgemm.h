@@ -134,11 +134,13 @@ typedef struct {
                                    allowed and only slower).  The first 64 KiB are a header in which only the
                                    weight-streaming kernel's arrival words ever live; the buffer need not be cleared,
                                    and launches that may overlap on the GPU need separate buffers */
-    int b_is_static;            /* non-zero: B and its scale bytes were complete before the kernel that precedes
-                                   this call in the stream was launched (a pre-packed weight).  The weight-streaming
-                                   kernel is launched with programmatic stream serialisation and then starts
-                                   fetching B while that predecessor (e.g. the activation quantiser) still runs;
-                                   A, its scales and every output are touched only after the predecessor is done. */
+    int b_is_static;            /* non-zero: B and its scale bytes are not written by the kernel that precedes this
+                                   call in the stream (a pre-packed weight).  The weight-streaming kernel is launched
+                                   with programmatic stream serialisation and then starts fetching B while that
+                                   predecessor (e.g. the activation quantiser) still runs; A, its scales and every
+                                   output are touched only after the predecessor is done.  What earlier kernels wrote
+                                   is complete by then: every kernel of this library lets its successor start only
+                                   after its own predecessor has completed. */
     int activation;             /* DSL_ACT_NONE, or DSL_ACT_SWIGLU / DSL_ACT_GEGLU: the GEMM's columns are (gate, up) pairs - column 2j
                                    is gate_j, column 2j+1 is up_j, i.e. the weight rows were interleaved when it was
                                    packed - and C is [M_total, N/2] with C[m,j] = silu(gate) * up computed in fp32 on
