@@ -65,7 +65,10 @@ extern "C" int dsl_linear(const void* x, int x_dtype, long long M, const dsl_wei
     if (w->groups > 1 && group_offsets == nullptr) return DSL_ERR_NULL;
     const int* offs = w->groups > 1 ? group_offsets : nullptr;
     dsl_epilogue e = *ep;
-    e.b_is_static = 1;                      // a packed weight is complete long before this call
+    // The activation quantiser stands between the weight's producer and the GEMM, so the weight is complete before the GEMM's
+    // predecessor starts.  BF16 has no quantiser: its weight may be the result of the very kernel before this call (a bf16
+    // result used as it lies, a weight packed a moment ago), so there the caller's word decides.
+    e.b_is_static = w->format == DSL_W_BF16 ? ep->b_is_static : 1;
     if (w->format == DSL_W_BF16) {
         if (x_dtype != DSL_BF16) return DSL_ERR_ENUM;
         return dsl_gemm_bf16(x, w->q, C, ldc, M, w->n, w->k, offs, w->groups, &e, status, stream);

@@ -384,8 +384,9 @@ def linear(a: torch.Tensor, w: PackedWeight, *, out_dtype=torch.float32,
            expert_offsets: Optional[torch.Tensor] = None, row_scale=None, col_scale=None,
            activation: Optional[str] = None, out_global_scale: Scalar = None, act_global_scale: Scalar = None):
     """a [M, K] high-precision activations x packed weight -> [M, N]: quantise the activations
-    in the weight's format (one pass on the GPU) and run the matching GEMM.  The packed weight is
-    treated as complete (the activation quantiser always sits between its producer and the GEMM).
+    in the weight's format (one pass on the GPU) and run the matching GEMM.  A weight of a
+    quantised format may be fetched while the activation quantiser still runs (which stands between the weight's
+    producer and the GEMM); a bf16 one, which has no quantiser before it, is read only when the kernel before this call is done.
     activation "swiglu" / "geglu": the weight is a fused gate/up projection packed with `gate_up_interleave=True`;
     the result is [M, N/2] = silu(gate) * up (gelu(gate) * up, tanh form), computed in the GEMM epilogue
     (cuda/activations/fused_gated_activations.cu:75-90 without the [M, N] round trip through memory).
