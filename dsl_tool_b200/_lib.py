@@ -203,40 +203,19 @@ def scratch_word(device: torch.device) -> torch.Tensor:
     return t
 
 
-_workspace: Dict[tuple, torch.Tensor] = {}
-_retired_workspaces: list = []
 WORKSPACE_BYTES = 16 << 20
 
 
-def workspace(device: torch.device, need: int = WORKSPACE_BYTES) -> Optional[torch.Tensor]:
-    """Scratch for partial sums along K, one buffer per (device, stream): launches on one stream use
-    it in order, launches on different streams never share it.  `need` is what dsl_workspace_bytes()
-    reports for the problem: 0 gives None (the kernels serving it use no scratch), anything else a
-    buffer of at least that size (it only ever grows)."""
-    if need <= 0:
-        return None
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, torch.cuda.current_stream(device).cuda_stream)
-    t = _workspace.get(key)
-    if t is None or t.numel() < need:
-        if torch.cuda.is_current_stream_capturing():
-            # memory allocated under capture belongs to that graph's pool: the caller holds it for this call only
-            return torch.empty(int(need), dtype=torch.uint8, device=device)
-        if t is not None:
-            _retired_workspaces.append(t)      # a captured CUDA graph may still point at it
-        # powers of two, so that what a stream has outgrown adds up to less than what it has
-        t = torch.empty(max(1 << (int(need) - 1).bit_length(), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
-        _workspace[key] = t
-    return t
-
-
-class ActArena:
-    """Scratch for the quantised activations of `dsl_linear`, one per (device, stream).  The GEMM of a call
-    consumes what the quantiser of the same call wrote, so calls issued in order on one stream share it; the
-    lock keeps two host threads that launch on the same stream from interleaving their two launches."""
+class StreamScratch:
+    """Device memory that the calls issued on one (device, stream) share: the quantised activations of `dsl_linear` and the
+    workspace for partial sums along K.  What a call leaves there is consumed by a later launch of the same call, so
+    calls issued in order on one stream need no more than this; launches on other streams never share it.  `lock` is held
+    from taking a buffer to the last launch that uses it: it keeps two host threads that launch on the same stream from
+    interleaving their launches."""
 
     def __init__(self) -> None:
-        self.buf: Optional[torch.Tensor] = None
+        self.buf: Optional[torch.Tensor] = None          # quantised activations
+        self.ws: Optional[torch.Tensor] = None           # partial sums
         self.lock = threading.Lock()
         self.retired: list = []      # outgrown buffers stay alive: a captured CUDA graph may still point at them
 
@@ -252,16 +231,32 @@ class ActArena:
             self.buf = buf
         return buf
 
+    def workspace(self, device: torch.device, need: int) -> Optional[torch.Tensor]:
+        """`need` is what dsl_workspace_bytes() reports for the problem: 0 gives None (the kernels serving it use no scratch),
+        anything else a buffer of at least that size (it only ever grows)."""
+        if need <= 0:
+            return None
+        ws = self.ws
+        if ws is None or ws.numel() < need:
+            if torch.cuda.is_current_stream_capturing():
+                return torch.empty(need, dtype=torch.uint8, device=device)
+            if ws is not None:
+                self.retired.append(ws)
+            # powers of two, so that what a stream has outgrown adds up to less than what it has
+            ws = torch.empty(max(1 << (need - 1).bit_length(), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
+            self.ws = ws
+        return ws
 
-_arenas: Dict[tuple, ActArena] = {}
+
+_stream_scratch: Dict[tuple, StreamScratch] = {}
 
 
-def act_arena(device: torch.device, stream: int) -> ActArena:
+def act_arena(device: torch.device, stream: int) -> StreamScratch:
     key = (device.index, stream)
-    a = _arenas.get(key)
+    a = _stream_scratch.get(key)
     if a is None:
         with _lock:
-            a = _arenas.setdefault(key, ActArena())
+            a = _stream_scratch.setdefault(key, StreamScratch())
     return a
 
 

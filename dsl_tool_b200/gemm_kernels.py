@@ -91,9 +91,7 @@ def _make_output(dev, M: int, nc: int, out_dtype, out_global_scale: Scalar, offs
 
 def _epilogue(dev, scale_a: Scalar, scale_b: Scalar, out: torch.dtype,
               row_scale: Optional[torch.Tensor], col_scale: Optional[torch.Tensor], keep: list,
-              b_static: bool = False, activation: Optional[str] = None, problem: Optional[tuple] = None) -> _lib.Epilogue:
-    """`problem` = (DSL_OP_* code, M, N, K, groups): the scratch the kernels can use for it is asked
-    from the library (dsl_workspace_bytes) and attached; without it no scratch is passed."""
+              b_static: bool = False, activation: Optional[str] = None) -> _lib.Epilogue:
     ep = _lib.Epilogue()
     ep.b_is_static = 1 if b_static else 0
     ep.activation = _activation_code(activation)
@@ -115,14 +113,24 @@ def _epilogue(dev, scale_a: Scalar, scale_b: Scalar, out: torch.dtype,
             keep.append(t)
             setattr(ep, name, t.data_ptr())
     ep.out_dtype = _lib.F32 if out in (None, torch.float32) else _lib.BF16
-    if problem is not None:
-        with torch.cuda.device(dev):
-            ws = _lib.workspace(dev, int(_lib.lib().dsl_workspace_bytes(*problem)))
-        if ws is not None:
-            keep.append(ws)
+    return ep
+
+
+def _run(dev, ep: "_lib.Epilogue", problem: tuple, launch) -> int:
+    """One GEMM entry point: `launch(status, stream)` -> return code.  `problem` = (DSL_OP_* code, M, N, K, groups): the
+    scratch that the kernels can use for it (dsl_workspace_bytes) is the current stream's, and its lock is held over
+    the call, whose launches hand sums to one another through it."""
+    with torch.cuda.device(dev):
+        status, stream = _lib.status_word(dev).data_ptr(), _lib.stream_ptr()
+        need = int(_lib.lib().dsl_workspace_bytes(*problem))
+        if need <= 0:
+            return launch(status, stream)
+        scratch = _lib.act_arena(dev, stream)
+        with scratch.lock:
+            ws = scratch.workspace(dev, need)
             ep.workspace = ws.data_ptr()
             ep.workspace_bytes = ws.numel()
-    return ep
+            return launch(status, stream)
 
 
 def _bytes2d(t: torch.Tensor) -> torch.Tensor:
@@ -169,13 +177,11 @@ def gemm_fp8_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, scale_a: Scalar, s
         raise ValueError(f"weight must be [{groups}*{n}, {K}] K-major bytes, got {tuple(qb_nk.shape)}")
     nc = _out_cols(n, activation)
     keep: list = []
-    ep = _epilogue(dev, scale_a, scale_b, None, row_scale, col_scale, keep, b_static, activation,
-                   (_lib.OP_GEMM_FP8, M, n, K, groups))
+    ep = _epilogue(dev, scale_a, scale_b, None, row_scale, col_scale, keep, b_static, activation)
     ep.b_is_kn = 1 if b_kn else 0
     out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_gemm_fp8(qa.data_ptr(), qb_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
-                                     groups, ctypes.byref(ep), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+    rc = _run(dev, ep, (_lib.OP_GEMM_FP8, M, n, K, groups), lambda status, stream: _lib.lib().dsl_gemm_fp8(
+        qa.data_ptr(), qb_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs), groups, ctypes.byref(ep), status, stream))
     _lib.check(rc, "dsl_gemm_fp8")
     return ret
 
@@ -207,14 +213,11 @@ def gemm_fp8_groupwise_quantized(qa: torch.Tensor, qb_nk: torch.Tensor, sa: torc
     nc = _out_cols(n, activation)
     out = torch.empty((M, nc), dtype=_out_dtype(out_dtype), device=dev)
     keep: list = []
-    ep = _epilogue(dev, None, None, out.dtype, row_scale, col_scale, keep, False, activation,
-                   (_lib.OP_GEMM_FP8_GROUPWISE, M, n, K, groups))
+    ep = _epilogue(dev, None, None, out.dtype, row_scale, col_scale, keep, False, activation)
     ep.b_is_kn = 1 if b_kn else 0
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_gemm_fp8_groupwise(qa.data_ptr(), qb_nk.data_ptr(), sa.data_ptr(), sb.data_ptr(),
-                                               1 if sb_block else 0, out.data_ptr(), nc, M, n, K, _lib.ptr(offs),
-                                               groups, ctypes.byref(ep), _lib.status_word(dev).data_ptr(),
-                                               _lib.stream_ptr())
+    rc = _run(dev, ep, (_lib.OP_GEMM_FP8_GROUPWISE, M, n, K, groups), lambda status, stream: _lib.lib().dsl_gemm_fp8_groupwise(
+        qa.data_ptr(), qb_nk.data_ptr(), sa.data_ptr(), sb.data_ptr(), 1 if sb_block else 0, out.data_ptr(), nc, M, n, K,
+        _lib.ptr(offs), groups, ctypes.byref(ep), status, stream))
     _lib.check(rc, "dsl_gemm_fp8_groupwise")
     return out
 
@@ -252,13 +255,13 @@ def gemm_fp4_quantized(pa: torch.Tensor, pb_nk: torch.Tensor, sfa: torch.Tensor,
         if token_scale.numel() != M:
             raise ValueError(f"token_scale must have {M} elements, got {token_scale.numel()}")
         row_scale = token_scale
-    ep = _epilogue(dev, global_scale_a, global_scale_b, None, row_scale, col_scale, keep, b_static, activation,
-                   (_lib.OP_GEMM_FP4_NV if fmt == _lib.FP4_NV else _lib.OP_GEMM_FP4_MX, M, n, K, groups))
+    ep = _epilogue(dev, global_scale_a, global_scale_b, None, row_scale, col_scale, keep, b_static, activation)
     out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_gemm_fp4(pa.data_ptr(), pb_nk.data_ptr(), _bytes2d(sfa).data_ptr(),
-                                     _bytes2d(sfb).data_ptr(), fmt, out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
-                                     groups, ctypes.byref(ep), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+    sfa, sfb = _bytes2d(sfa), _bytes2d(sfb)
+    op = _lib.OP_GEMM_FP4_NV if fmt == _lib.FP4_NV else _lib.OP_GEMM_FP4_MX
+    rc = _run(dev, ep, (op, M, n, K, groups), lambda status, stream: _lib.lib().dsl_gemm_fp4(
+        pa.data_ptr(), pb_nk.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), fmt, out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
+        groups, ctypes.byref(ep), status, stream))
     _lib.check(rc, "dsl_gemm_fp4")
     return ret
 
@@ -275,12 +278,11 @@ def gemm_bf16_raw(a: torch.Tensor, b_nk: torch.Tensor, *, n: int, out_dtype=torc
         raise ValueError(f"weight must be [{groups}*{n}, {K}] K-major, got {tuple(b_nk.shape)}")
     nc = _out_cols(n, activation)
     keep: list = []
-    ep = _epilogue(dev, scale_a, scale_b, None, None, None, keep, False, activation, (_lib.OP_GEMM_BF16, M, n, K, groups))
+    ep = _epilogue(dev, scale_a, scale_b, None, None, None, keep, False, activation)
     ep.b_is_kn = 1 if b_kn else 0
     out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_gemm_bf16(a.data_ptr(), b_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs),
-                                      groups, ctypes.byref(ep), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+    rc = _run(dev, ep, (_lib.OP_GEMM_BF16, M, n, K, groups), lambda status, stream: _lib.lib().dsl_gemm_bf16(
+        a.data_ptr(), b_nk.data_ptr(), out.data_ptr(), ldc, M, n, K, _lib.ptr(offs), groups, ctypes.byref(ep), status, stream))
     _lib.check(rc, "dsl_gemm_bf16")
     return ret
 
@@ -355,11 +357,8 @@ def _linear_one_call(a: torch.Tensor, w: PackedWeight, out_dtype, offs: Optional
         prev = torch.cuda.current_device()
         torch.cuda.set_device(dev)
     try:
-        if groups == 1:                    # row groups never use scratch; the library says what a dense problem can use
-            ws = _lib.workspace(dev, int(lib.dsl_workspace_bytes(_OP_OF_FORMAT[w.format], M, w.n, w.k, 1)))
-            if ws is not None:
-                ep.workspace = ws.data_ptr()
-                ep.workspace_bytes = ws.numel()
+        # row groups never use a workspace; the library says what a dense problem can use
+        ws_need = int(lib.dsl_workspace_bytes(_OP_OF_FORMAT[w.format], M, w.n, w.k, 1)) if groups == 1 else 0
         out, ldc, ret = _make_output(dev, M, nc, out_dtype, out_global_scale, offs, groups, ep, keep)
         need = w._scratch_need.get(M)
         if need is None:
@@ -367,9 +366,13 @@ def _linear_one_call(a: torch.Tensor, w: PackedWeight, out_dtype, offs: Optional
             if len(w._scratch_need) < 64:
                 w._scratch_need[M] = need
         stream = torch.cuda.current_stream(dev).cuda_stream
-        arena = _lib.act_arena(dev, stream)
-        with arena.lock:
-            buf = arena.get(dev, need) if need else None
+        scratch = _lib.act_arena(dev, stream)
+        with scratch.lock:
+            buf = scratch.get(dev, need) if need else None
+            ws = scratch.workspace(dev, ws_need)
+            if ws is not None:
+                ep.workspace = ws.data_ptr()
+                ep.workspace_bytes = ws.numel()
             rc = lib.dsl_linear(a.data_ptr(), _lib.dtype_code(a.dtype), M, ctypes.byref(desc), _lib.ptr(offs),
                                 _lib.ptr(buf), 0 if buf is None else buf.numel(), out.data_ptr(), ldc, ctypes.byref(ep),
                                 _lib.status_word(dev).data_ptr(), stream)
