@@ -180,7 +180,6 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 _status: Dict[int, torch.Tensor] = {}
-_scratch: Dict[int, torch.Tensor] = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -193,22 +192,12 @@ def status_word(device: torch.device) -> torch.Tensor:
     return t
 
 
-def scratch_word(device: torch.device) -> torch.Tensor:
-    """Per-device 16-byte scratch (tensor amax cell)."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    t = _scratch.get(idx)
-    if t is None:
-        t = torch.zeros(4, dtype=torch.int32, device=device)
-        _scratch[idx] = t
-    return t
-
-
 WORKSPACE_BYTES = 16 << 20
 
 
 class StreamScratch:
-    """Device memory that the calls issued on one (device, stream) share: the quantised activations of `dsl_linear` and the
-    workspace for partial sums along K.  What a call leaves there is consumed by a later launch of the same call, so
+    """Device memory that the calls issued on one (device, stream) share: the quantised activations of `dsl_linear`, the
+    workspace for partial sums along K and the cell for a tensor's amax.  What a call leaves there is consumed by a later launch of the same call, so
     calls issued in order on one stream need no more than this; launches on other streams never share it.  `lock` is held
     from taking a buffer to the last launch that uses it: it keeps two host threads that launch on the same stream from
     interleaving their launches."""
@@ -216,6 +205,7 @@ class StreamScratch:
     def __init__(self) -> None:
         self.buf: Optional[torch.Tensor] = None          # quantised activations
         self.ws: Optional[torch.Tensor] = None           # partial sums
+        self.cell: Optional[torch.Tensor] = None         # amax of the tensor being quantised
         self.lock = threading.Lock()
         self.retired: list = []      # outgrown buffers stay alive: a captured CUDA graph may still point at them
 
@@ -246,6 +236,14 @@ class StreamScratch:
             ws = torch.empty(max(1 << (need - 1).bit_length(), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
             self.ws = ws
         return ws
+
+
+    def amax_cell(self, device: torch.device) -> torch.Tensor:
+        if self.cell is None:
+            if torch.cuda.is_current_stream_capturing():
+                return torch.empty(4, dtype=torch.int32, device=device)
+            self.cell = torch.empty(4, dtype=torch.int32, device=device)
+        return self.cell
 
 
 _stream_scratch: Dict[tuple, StreamScratch] = {}

@@ -26,6 +26,19 @@ def _as_2d(x: torch.Tensor) -> torch.Tensor:
     return x.contiguous()
 
 
+def _with_amax_cell(dev: torch.device, wanted: bool, launch) -> int:
+    """`launch(cell, stream)` -> return code of a quantiser; `wanted`: it takes the tensor's amax first, in launches of their
+    own that leave it in the stream's cell, so the stream's lock is held over the call."""
+    with torch.cuda.device(dev):
+        stream = _lib.stream_ptr()
+        if not wanted:
+            return launch(None, stream)
+        scratch = _lib.act_arena(dev, stream)
+        with scratch.lock:
+            cell = scratch.amax_cell(dev)
+            return launch(cell.data_ptr(), stream)
+
+
 def quantize_fp8(x: torch.Tensor, mode: str = "per_tensor",
                  scale: Union[None, float, torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """x [rows, cols] (float32 / bfloat16 / float16, CUDA) -> (E4M3 bytes [rows, cols] uint8, scales fp32).
@@ -52,10 +65,8 @@ def quantize_fp8(x: torch.Tensor, mode: str = "per_tensor",
         s = torch.empty((rows, (cols + 127) // 128), dtype=torch.float32, device=dev)
     else:
         s = torch.empty(((rows + 127) // 128, (cols + 127) // 128), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_quant_fp8(x.data_ptr(), _lib.dtype_code(x.dtype), rows, cols, FP8_MODES[mode],
-                                      s.data_ptr(), given, q.data_ptr(), _lib.scratch_word(dev).data_ptr(),
-                                      _lib.stream_ptr())
+    rc = _with_amax_cell(dev, mode == "per_tensor" and not given, lambda cell, stream: _lib.lib().dsl_quant_fp8(
+        x.data_ptr(), _lib.dtype_code(x.dtype), rows, cols, FP8_MODES[mode], s.data_ptr(), given, q.data_ptr(), cell, stream))
     _lib.check(rc, "dsl_quant_fp8")
     return q, s
 
@@ -117,11 +128,9 @@ def quantize_fp4(x: torch.Tensor, format: str = "nvfp4",
                   if isinstance(global_scale, torch.Tensor)
                   else torch.full((1,), float(global_scale), dtype=torch.float32, device=dev))
             given = 1
-    with torch.cuda.device(dev):
-        rc = _lib.lib().dsl_quant_fp4(x.data_ptr(), _lib.dtype_code(x.dtype), rows, cols, FP4_FORMATS[format],
-                                      _lib.ptr(gs), given, q.data_ptr(), sf.data_ptr(),
-                                      _lib.ptr(group_offsets), groups, _lib.scratch_word(dev).data_ptr(),
-                                      _lib.stream_ptr())
+    rc = _with_amax_cell(dev, format == "nvfp4" and not given, lambda cell, stream: _lib.lib().dsl_quant_fp4(
+        x.data_ptr(), _lib.dtype_code(x.dtype), rows, cols, FP4_FORMATS[format], _lib.ptr(gs), given, q.data_ptr(), sf.data_ptr(),
+        _lib.ptr(group_offsets), groups, cell, stream))
     _lib.check(rc, "dsl_quant_fp4")
     return q, sf, gs
 

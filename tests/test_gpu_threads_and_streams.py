@@ -1,5 +1,5 @@
 """Host threads that launch on one stream, and streams side by side, against the same calls one after the other, with ==: problems
-whose sums along K pass through the stream's scratch between two launches."""
+whose sums along K pass through the stream's scratch between two launches, and tensor-wide scales, whose amax does."""
 import threading
 
 import pytest
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 def _calls():
     """(name, call) on operands of its own: dense problems of few tiles, which the CTA-pair kernels cut along K, a narrow output
     on the 1-CTA kernel and a decode shape of more column tiles than SMs."""
-    from dsl_tool_b200 import bf16_gemm, fp8_gemm, linear, pack_weight
+    from dsl_tool_b200 import bf16_gemm, fp8_gemm, linear, pack_weight, quantize_fp4, quantize_fp8
     gen = torch.Generator(device="cuda").manual_seed(3)
     def draw(*shape):
         return torch.randn(shape, generator=gen, device="cuda")
@@ -22,7 +22,8 @@ def _calls():
     x, xd = draw(256, 8192).bfloat16(), draw(20, 1024).bfloat16()
     return {"bf16": lambda: bf16_gemm(a, b), "fp8": lambda: fp8_gemm(qa, qb, 0.01, 0.02),
             "fp8_groupwise": lambda: fp8_gemm(qa, qb, ga, gb, mode="groupwise"), "nvfp4": lambda: linear(x, w4),
-            "narrow": lambda: linear(x, wn), "decode": lambda: linear(xd, wd)}
+            "narrow": lambda: linear(x, wn), "decode": lambda: linear(xd, wd),
+            "quantize_fp8": lambda: quantize_fp8(a)[1], "quantize_fp4": lambda: quantize_fp4(b)[2]}
 
 
 def _side_by_side(calls, streams):

@@ -9,12 +9,12 @@ import types
 import pytest
 import torch
 
-from dsl_tool_b200 import _lib, gemm_kernels
+from dsl_tool_b200 import _lib, gemm_kernels, quantize
 from dsl_tool_b200.quantize import PackedWeight
 
 
 class FakeLibrary:
-    """Every dsl_gemm_* / dsl_linear records which calls are inside with the same workspace at the same time."""
+    """Every dsl_gemm_* / dsl_linear / dsl_quant_* records which calls are inside with the same scratch at the same time."""
 
     def __init__(self):
         self.inside, self.overlaps, self.workspaces, self.guard = {}, 0, set(), threading.Lock()
@@ -24,16 +24,20 @@ class FakeLibrary:
             return lambda *problem: 1 << 16
         if name == "dsl_linear_scratch_bytes":
             return lambda *args: 1 << 12
-        return lambda *args: self._call([a._obj for a in args if isinstance(getattr(a, "_obj", None), _lib.Epilogue)][0])
+        if name.startswith("dsl_sf_bytes"):
+            return lambda *args: 512
+        if name.startswith("dsl_quant"):
+            return lambda *args: self._call(args[-2])           # ws, stream
+        return lambda *args: self._call([a._obj for a in args if isinstance(getattr(a, "_obj", None), _lib.Epilogue)][0].workspace)
 
-    def _call(self, ep):
+    def _call(self, scratch):
         with self.guard:
-            self.overlaps += self.inside.get(ep.workspace, 0)
-            self.inside[ep.workspace] = self.inside.get(ep.workspace, 0) + 1
-            self.workspaces.add(ep.workspace)
+            self.overlaps += self.inside.get(scratch, 0)
+            self.inside[scratch] = self.inside.get(scratch, 0) + 1
+            self.workspaces.add(scratch)
         time.sleep(0.002)
         with self.guard:
-            self.inside[ep.workspace] -= 1
+            self.inside[scratch] -= 1
         return 0
 
 
@@ -91,3 +95,12 @@ def test_streams_have_workspaces_of_their_own(fake):
     calls = _calls()
     _together(calls, before=lambda i: setattr(fake.streams, "value", 100 + i))
     assert fake.overlaps == 0 and len(fake.workspaces) == len(calls)
+
+
+@pytest.mark.parametrize("one_stream", [True, False])
+def test_the_amax_cell_of_the_quantisers(fake, one_stream):
+    """Per-tensor FP8 and NVFP4 scales: the amax pass and the quantise pass of a call meet in a cell of the stream."""
+    x = torch.zeros((8, 64))
+    calls = [lambda: quantize.quantize_fp8(x), lambda: quantize.quantize_fp4(x)] * 2
+    _together(calls, before=lambda i: setattr(fake.streams, "value", 100 + (0 if one_stream else i)))
+    assert fake.overlaps == 0 and len(fake.workspaces) == (1 if one_stream else 4) and None not in fake.workspaces
