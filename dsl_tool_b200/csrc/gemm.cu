@@ -407,6 +407,10 @@ bool make_tmap_u8(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, ui
     }
     EncodeTiledFn enc = get_encoder();
     if (enc == nullptr) return false;
+    // The encoder wants a current context, and a host thread whose first CUDA work this call is has none yet (asking for the
+    // device does not make one).
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return false;
     cuuint64_t dims[3] = {d0, d1, d2};
     cuuint64_t strides[2] = {d0, d0 * d1};
     cuuint32_t box[3] = {box0, box1, 1};

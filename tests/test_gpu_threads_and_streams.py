@@ -32,10 +32,13 @@ def _side_by_side(calls, streams):
     wrong = []
 
     def work(name, call, stream):
-        with torch.cuda.stream(stream):
-            results = [call() for _ in range(30)]
-            stream.synchronize()
-        wrong.extend(name for r in results if not torch.equal(r, want[name]))
+        try:
+            with torch.cuda.stream(stream):
+                results = [call() for _ in range(30)]
+                stream.synchronize()
+            wrong.extend(name for r in results if not torch.equal(r, want[name]))
+        except Exception as e:          # an exception in a thread would be lost
+            wrong.append(f"{name}: {e!r}")
     threads = [threading.Thread(target=work, args=(name, call, streams(i))) for i, (name, call) in enumerate(calls.items())]
     for t in threads:
         t.start()
@@ -53,3 +56,17 @@ def test_threads_on_one_stream(cuda_device):
 
 def test_a_stream_for_every_thread(cuda_device):
     _side_by_side(_calls(), lambda i: torch.cuda.Stream())
+
+
+@pytest.mark.parametrize("name", ["bf16", "fp8", "fp8_groupwise", "nvfp4", "narrow", "decode"])
+def test_first_cuda_work_of_a_thread(cuda_device, name):
+    """Nothing before the GEMM has given the host thread a context: operands and result come from the allocator's cache."""
+    call = _calls()[name]
+    want = call()
+    call()
+    torch.cuda.synchronize()
+    got = []
+    thread = threading.Thread(target=lambda: got.append(call()))
+    thread.start()
+    thread.join()
+    assert len(got) == 1 and torch.equal(got[0], want)
