@@ -570,6 +570,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                         const int row = c * 4 + i;
                         if (row < args.m_total) store_out(args, row, col, __uint_as_float(v[i]), s1, s2, cs, col_ok);
                     }
+                    __syncwarp();            // lanes leave store_out apart; the next load from tensor memory takes the whole warp
                 }
                 tc_fence_before();
                 __syncwarp();

@@ -28,6 +28,7 @@ __device__ __forceinline__ bool promote_run(const float* __restrict__ sa_rows, i
     constexpr int J = (TOK + 31) / 32;
     constexpr int DEPTH = TOK > 64 ? 2 : 4;
     float sa_q[DEPTH][J], sb_q[DEPTH];
+    __syncwarp();       // `tscale` restarts at its first buffer: the last reads of the run before (any length) are behind every lane
     auto fetch = [&](int i, float (&sa)[J], float& sb) {
         int kb = i + rot;
         if (kb >= len) kb -= len;
