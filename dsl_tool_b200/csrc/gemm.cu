@@ -551,7 +551,7 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args) {
         const size_t b = decode_scratch_bytes(kind, args, &served);
         if (served) return b > 0 ? b + DSL_WS_HEADER_BYTES : 0;
     }
-    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) {
+    if (forced == 2 || (forced == 0 && pair_shape(args.m_total, args.n))) {
         const int s = choose_pair_split(kind, args);
         return s > 1 ? DSL_WS_HEADER_BYTES + static_cast<size_t>(s) * args.m_total * args.n * sizeof(float) : 0;
     }
@@ -573,7 +573,7 @@ bool kn_served(int kind, const GemmArgs& args) {
     if (args.n <= 0 || args.m_total <= 0 || (static_cast<long long>(args.n) * elem) % 16 != 0 || forced_kernel() != 0) return false;
     bool decode = false;
     decode_scratch_bytes(kind, args, &decode);
-    return decode || decode_grouped_served(args) || (args.m_total > 128 && args.n >= 256);
+    return decode || decode_grouped_served(args) || pair_shape(args.m_total, args.n);
 }
 
 int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStream_t st) {
@@ -584,7 +584,7 @@ int launch_gemm(int kind, const void* A, const void* B, GemmArgs args, cudaStrea
         if (rc == DSL_NOT_SERVED) rc = launch_gemm_decode_grouped(kind, A, B, args, st);
         if (rc != DSL_NOT_SERVED) return rc;
     }
-    if (forced == 2 || (forced == 0 && args.m_total > 128 && args.n >= 256)) {
+    if (forced == 2 || (forced == 0 && pair_shape(args.m_total, args.n))) {
         args.split_k = choose_pair_split(kind, args);
         return launch_gemm_pair(kind, A, B, args, st);
     }

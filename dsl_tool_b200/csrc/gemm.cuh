@@ -85,6 +85,8 @@ size_t gemm_workspace_bytes(int kind, const GemmArgs& args);
 // Whether a problem whose B is stored [K, N] can be multiplied without transposing B first (the CTA-pair kernels and the
 // weight-streaming kernel read it MN-major; the 1-CTA kernels do not).
 bool kn_served(int kind, const GemmArgs& args);
+// Shapes of the CTA-pair kernels: more than one 128-row tile of work and an output at least one of their tiles wide.
+inline bool pair_shape(long long m_total, int n) { return m_total > 128 && n >= 256; }
 int choose_split_k(const GemmArgs& args, long long tiles);
 int choose_pair_split(int kind, const GemmArgs& args);
 int launch_splitk_reduce(const GemmArgs& args, cudaStream_t st);

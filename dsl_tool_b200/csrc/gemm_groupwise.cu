@@ -256,7 +256,7 @@ int launch_gemm_fp8_groupwise(const void* A, const void* B, GemmArgs args, cudaS
         if (rc == DSL_NOT_SERVED) rc = launch_gemm_decode_grouped(KIND_F8G, A, B, args, st);
         if (rc != DSL_NOT_SERVED) return rc;
     }
-    if (!force_1cta && args.m_total > 128 && args.n >= 256) return launch_gemm_fp8_groupwise_pair(A, B, args, st);
+    if (!force_1cta && pair_shape(args.m_total, args.n)) return launch_gemm_fp8_groupwise_pair(A, B, args, st);
     if (args.band <= 0) args.band = 8;
     // two instantiations: the plain epilogue keeps the promotion loop free of spills, the activation one is larger
     if (args.act != DSL_ACT_NONE)

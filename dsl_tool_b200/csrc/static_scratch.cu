@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "dslgemm.h"
+#include "gemm.cuh"
 
 // Held by every GPU that loads the library, until the process exits.
 static __device__ __align__(256) unsigned char g_static_scratch[DSL_STATIC_SCRATCH_BYTES];
@@ -46,6 +47,12 @@ extern "C" int dsl_gemm_fp4_static_scratch(const uint8_t* A, const uint8_t* B, c
     if (ep == nullptr) return DSL_ERR_NULL;
     if (M < 0 || N < 0 || K <= 0) return DSL_ERR_SHAPE;
     if (format != DSL_FP4_NV && format != DSL_FP4_MX) return DSL_ERR_ENUM;
+    dsl_epilogue local = *ep;
+    local.workspace = nullptr;
+    local.workspace_bytes = 0;
+    // The CTA-pair kernels need no scratch; what they could use it for (cutting K when they have few tiles) would not fit the
+    // array for most problems, and would make calls on several streams race on it.
+    if (dsl::pair_shape(M, N)) return dsl_gemm_fp4(A, B, sfa, sfb, format, C, ldc, M, N, K, nullptr, 1, &local, status, stream);
     // what the kernels serving this problem would take from a workspace must fit the array
     if (dsl_workspace_bytes(format == DSL_FP4_NV ? DSL_OP_GEMM_FP4_NV : DSL_OP_GEMM_FP4_MX, M, N, K, 1) >
         static_cast<size_t>(DSL_STATIC_SCRATCH_BYTES))
@@ -53,7 +60,6 @@ extern "C" int dsl_gemm_fp4_static_scratch(const uint8_t* A, const uint8_t* B, c
     void* scratch = nullptr;
     cudaError_t e = scratch_address(&scratch);
     if (e != cudaSuccess) return static_cast<int>(e);
-    dsl_epilogue local = *ep;
     local.workspace = scratch;
     local.workspace_bytes = DSL_STATIC_SCRATCH_BYTES;
     return dsl_gemm_fp4(A, B, sfa, sfb, format, C, ldc, M, N, K, nullptr, 1, &local, status, stream);

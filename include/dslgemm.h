@@ -347,7 +347,8 @@ int dsl_moe_unpack_wire_fp4(const uint8_t* wire_in, const int* ids, const int* d
  * ep->workspace (which is ignored), so nothing but inputs and outputs is passed and the call
  * performs no allocation.  Meant for decode-sized problems: it returns DSL_ERR_TOO_LARGE when
  * dsl_workspace_bytes() for the problem exceeds the array (e.g. 32 tokens against more than
- * 126 x 128 columns on a 148-SM part); problems that need no scratch at all pass through.
+ * 126 x 128 columns on a 148-SM part); problems that need no scratch at all pass through, and so do those of more
+ * than 128 rows and at least 256 columns, which run without any (never cut along K).
  * The first call on each device looks up the array's device address (cudaGetSymbolAddress);
  * make that call before any stream capture.  All calls share the one array and it keeps the
  * previous call's contents.  Partial sums are always written by a call before that call reads
