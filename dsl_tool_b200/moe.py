@@ -31,7 +31,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .gemm_kernels import _new_weight_desc, gemm_fp4_quantized, gemm_fp8_groupwise_quantized, gemm_fp8_quantized, linear
+from .gemm_kernels import _BYTE_DTYPES, _new_weight_desc, gemm_fp4_quantized, gemm_fp8_groupwise_quantized, gemm_fp8_quantized, linear
 from .quantize import PackedWeight, pack_weight, quantize_fp4, quantize_fp8
 from .sharding import arrival_expert_ids, exchange_rows, expert_ranges, return_rows
 
@@ -192,16 +192,39 @@ def _experts_fp4(p: MoEPlan, packed: torch.Tensor, sf: torch.Tensor, gs, w: MoEW
                               global_scale_b=w.down.global_scale, out_dtype=torch.bfloat16, **common)
 
 
+def _plain(t: Optional[torch.Tensor], device: torch.device, dtypes) -> bool:
+    return t is not None and t.dtype in dtypes and t.device == device and t.is_contiguous()
+
+
+def _as_packed(w: PackedWeight, device: torch.device) -> bool:
+    """Whether the weight's tensors are what pack_weight makes for its format and sizes.  The one-call layer reads them by
+    pointer; anything else (assembled by hand) takes the step-by-step form, which checks or converts them."""
+    rows, q = w.groups * w.n, w.q
+    if w.format == "bf16":
+        return _plain(q, device, (torch.bfloat16,)) and q.shape == (rows, w.k)
+    fp4 = w.format in ("nvfp4", "mxfp4")
+    if not _plain(q, device, _BYTE_DTYPES) or q.shape != (rows, w.k // 2 if fp4 else w.k):
+        return False
+    tiles = w.groups * ((w.n + 127) // 128)
+    if not fp4:
+        return _plain(w.scale, device, (torch.float32,)) and w.scale.numel() == (1 if w.format == "fp8" else tiles * ((w.k + 127) // 128))
+    katoms = (w.k // (16 if w.format == "nvfp4" else 32) + 3) // 4
+    return (_plain(w.scale, device, _BYTE_DTYPES) and w.scale.numel() >= tiles * katoms * 512
+            and (w.format == "mxfp4" or (_plain(w.global_scale, device, (torch.float32,)) and w.global_scale.numel() == 1)))
+
+
 def _whole_layer(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, renormalize: bool, out_dtype,
                  act_global_scale) -> Optional[torch.Tensor]:
     """The layer through the single C entry point `dsl_moe_layer` (same launches, same bits as the steps below, without
     the host time between them), or None when that call does not take it: only part of the experts, shapes the packed
-    weights do not match, row lengths its dispatch cannot move."""
+    weights do not match, weights that are not as pack_weight lays them out, row lengths its dispatch cannot move."""
     gu, dn, hgs = w.gate_up, w.down, w.hidden_global_scale
     if (w.first != 0 or w.last != w.experts or gu.groups != w.experts or dn.groups != w.experts or gu.format != dn.format
             or x.dim() != 2 or logits.dim() != 2 or logits.shape != (x.shape[0], w.experts) or x.shape[0] == 0 or x.shape[1] != gu.k
             or logits.dtype not in (torch.float32, torch.bfloat16) or x.dtype not in (torch.float32, torch.bfloat16, torch.float16)
             or out_dtype not in (torch.float32, torch.bfloat16) or not 1 <= k <= min(32, w.experts)):
+        return None
+    if not (gu.gate_up_interleaved and _as_packed(gu, x.device) and _as_packed(dn, x.device)):
         return None
     fused = gu.format == "nvfp4" and hgs is not None
     if (fused and (isinstance(hgs, torch.Tensor) or not hgs > 0)) or isinstance(act_global_scale, str):
