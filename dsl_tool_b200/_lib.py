@@ -197,51 +197,46 @@ WORKSPACE_BYTES = 16 << 20
 
 class StreamScratch:
     """Device memory that the calls issued on one (device, stream) share: the quantised activations of `dsl_linear`, the
-    workspace for partial sums along K and the cell for a tensor's amax.  What a call leaves there is consumed by a later launch of the same call, so
-    calls issued in order on one stream need no more than this; launches on other streams never share it.  `lock` is held
-    from taking a buffer to the last launch that uses it: it keeps two host threads that launch on the same stream from
-    interleaving their launches."""
+    workspace for partial sums along K and the cell for a tensor's amax.  What a call leaves there is consumed by a later
+    launch of the same call, so calls issued in order on one stream need no more than this; launches on other streams never
+    share it.  `lock` is held from taking a buffer to the last launch that uses it: it keeps two host threads that launch on
+    the same stream from interleaving their launches.
+
+    A call under capture (`capturing`) gets memory of its own from the graph's pool (for that call only: the pool hands it to the next): the
+    graph may be replayed on any stream, beside the calls that share these buffers.  No graph points at them, so an outgrown
+    one goes back to the allocator, which keeps it for this stream."""
 
     def __init__(self) -> None:
         self.buf: Optional[torch.Tensor] = None          # quantised activations
         self.ws: Optional[torch.Tensor] = None           # partial sums
         self.cell: Optional[torch.Tensor] = None         # amax of the tensor being quantised
         self.lock = threading.Lock()
-        self.retired: list = []      # outgrown buffers stay alive: a captured CUDA graph may still point at them
 
-    def get(self, device: torch.device, need: int) -> torch.Tensor:
-        buf = self.buf
-        if buf is None or buf.numel() < need:
-            if torch.cuda.is_current_stream_capturing():
-                # memory allocated under capture belongs to that graph's pool: use it for this call only
-                return torch.empty(need, dtype=torch.uint8, device=device)
-            if buf is not None:
-                self.retired.append(buf)
-            buf = torch.empty(max(int(need * 1.25), 1 << 20), dtype=torch.uint8, device=device)
-            self.buf = buf
-        return buf
+    def get(self, device: torch.device, need: int, capturing: bool) -> torch.Tensor:
+        if capturing:
+            return torch.empty(need, dtype=torch.uint8, device=device)
+        if self.buf is None or self.buf.numel() < need:
+            self.buf = None
+            self.buf = torch.empty(max(int(need * 1.25), 1 << 20), dtype=torch.uint8, device=device)
+        return self.buf
 
-    def workspace(self, device: torch.device, need: int) -> Optional[torch.Tensor]:
+    def workspace(self, device: torch.device, need: int, capturing: bool) -> Optional[torch.Tensor]:
         """`need` is what dsl_workspace_bytes() reports for the problem: 0 gives None (the kernels serving it use no scratch),
         anything else a buffer of at least that size (it only ever grows)."""
         if need <= 0:
             return None
-        ws = self.ws
-        if ws is None or ws.numel() < need:
-            if torch.cuda.is_current_stream_capturing():
-                return torch.empty(need, dtype=torch.uint8, device=device)
-            if ws is not None:
-                self.retired.append(ws)
-            # powers of two, so that what a stream has outgrown adds up to less than what it has
-            ws = torch.empty(max(1 << (need - 1).bit_length(), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
-            self.ws = ws
-        return ws
+        if capturing:
+            return torch.empty(need, dtype=torch.uint8, device=device)
+        if self.ws is None or self.ws.numel() < need:
+            self.ws = None
+            # a quarter more than asked for, so that a run of growing problems does not allocate for each of them
+            self.ws = torch.empty(max(need + (need >> 2), WORKSPACE_BYTES), dtype=torch.uint8, device=device)
+        return self.ws
 
-
-    def amax_cell(self, device: torch.device) -> torch.Tensor:
+    def amax_cell(self, device: torch.device, capturing: bool) -> torch.Tensor:
+        if capturing:
+            return torch.empty(4, dtype=torch.int32, device=device)
         if self.cell is None:
-            if torch.cuda.is_current_stream_capturing():
-                return torch.empty(4, dtype=torch.int32, device=device)
             self.cell = torch.empty(4, dtype=torch.int32, device=device)
         return self.cell
 

@@ -125,9 +125,9 @@ def _run(dev, ep: "_lib.Epilogue", problem: tuple, launch) -> int:
         need = int(_lib.lib().dsl_workspace_bytes(*problem))
         if need <= 0:
             return launch(status, stream)
-        scratch = _lib.act_arena(dev, stream)
+        scratch, capturing = _lib.act_arena(dev, stream), torch.cuda.is_current_stream_capturing()
         with scratch.lock:
-            ws = scratch.workspace(dev, need)
+            ws = scratch.workspace(dev, need, capturing)
             ep.workspace = ws.data_ptr()
             ep.workspace_bytes = ws.numel()
             return launch(status, stream)
@@ -366,10 +366,10 @@ def _linear_one_call(a: torch.Tensor, w: PackedWeight, out_dtype, offs: Optional
             if len(w._scratch_need) < 64:
                 w._scratch_need[M] = need
         stream = torch.cuda.current_stream(dev).cuda_stream
-        scratch = _lib.act_arena(dev, stream)
+        scratch, capturing = _lib.act_arena(dev, stream), torch.cuda.is_current_stream_capturing()
         with scratch.lock:
-            buf = scratch.get(dev, need) if need else None
-            ws = scratch.workspace(dev, ws_need)
+            buf = scratch.get(dev, need, capturing) if need else None
+            ws = scratch.workspace(dev, ws_need, capturing)
             if ws is not None:
                 ep.workspace = ws.data_ptr()
                 ep.workspace_bytes = ws.numel()

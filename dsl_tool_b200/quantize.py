@@ -33,9 +33,9 @@ def _with_amax_cell(dev: torch.device, wanted: bool, launch) -> int:
         stream = _lib.stream_ptr()
         if not wanted:
             return launch(None, stream)
-        scratch = _lib.act_arena(dev, stream)
+        scratch, capturing = _lib.act_arena(dev, stream), torch.cuda.is_current_stream_capturing()
         with scratch.lock:
-            cell = scratch.amax_cell(dev)
+            cell = scratch.amax_cell(dev, capturing)
             return launch(cell.data_ptr(), stream)
 
 

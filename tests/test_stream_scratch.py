@@ -104,3 +104,22 @@ def test_the_amax_cell_of_the_quantisers(fake, one_stream):
     calls = [lambda: quantize.quantize_fp8(x), lambda: quantize.quantize_fp4(x)] * 2
     _together(calls, before=lambda i: setattr(fake.streams, "value", 100 + (0 if one_stream else i)))
     assert fake.overlaps == 0 and len(fake.workspaces) == (1 if one_stream else 4) and None not in fake.workspaces
+
+
+def test_captured_calls_share_nothing_and_outgrown_buffers_go(fake):
+    import gc
+    import weakref
+    scratch, cpu = _lib.StreamScratch(), torch.device("cpu")
+    buf, ws, cell = scratch.get(cpu, 1 << 20, False), scratch.workspace(cpu, 20 << 20, False), scratch.amax_cell(cpu, False)
+    assert scratch.get(cpu, 1 << 19, False) is buf and scratch.workspace(cpu, 1, False) is ws and scratch.amax_cell(cpu, False) is cell
+    assert scratch.workspace(cpu, 0, False) is None and ws.numel() < 2 * (20 << 20)
+    pointers = {t.data_ptr() for t in (buf, ws, cell)}
+    captured = [scratch.get(cpu, 1 << 10, True), scratch.workspace(cpu, 1 << 10, True), scratch.amax_cell(cpu, True)]
+    assert not pointers & {t.data_ptr() for t in captured}                  # a graph has memory of its own ...
+    assert scratch.buf is buf and scratch.ws is ws and scratch.cell is cell  # ... which calls outside it never see
+    old = [weakref.ref(buf), weakref.ref(ws)]
+    del buf, ws
+    scratch.get(cpu, 4 << 20, False)
+    scratch.workspace(cpu, 80 << 20, False)
+    gc.collect()
+    assert all(r() is None for r in old)
