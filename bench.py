@@ -9,7 +9,7 @@ public callable (`linear`).  The default workload is the FP8 groupwise GEMM at t
 shape (M=4096, K=4096, N=14336; 1x128 activation scales, 128x128 weight-block scales, bf16
 output).  Inputs are seeded synthetic tensors of the stated shapes and distributions.
 
-Prints ONE JSON line (rank 0).
+Prints ONE JSON line (rank 0), and to stderr one JSON object per sweep entry.
   * `value`: aggregate TFLOP/s over all ranks with inputs resident in HBM.  K steps are timed between
     two barriers with CUDA events, and that K-step block is repeated until the timed region lasts at
     least `--min-seconds` (default 1 s), so that the figure is taken at the clocks the part sustains;
@@ -18,7 +18,7 @@ Prints ONE JSON line (rank 0).
     timed blocks without a pause.
   * `e2e`: the same metric through the public callable with the activations in pinned host memory
     (host->device copy of the activations and device->host copy of the result inside the timed region).
-  * `sweep`: one short record per further configuration (decode shapes replayed as CUDA graphs).
+  * sweep (stderr): one record per further configuration (decode shapes replayed as CUDA graphs).
   * `cpu_baseline`: the reference's own CPU emulation (a copy made by `make -C oracle ref_py`) on a
     bounded slab of the workload, the numpy restatement beside it.
 With N > 1 the ONE problem is split across the ranks (`--scaling strong`, the default): 128-aligned
@@ -95,7 +95,7 @@ WORKLOADS = {
     "bf16_8192": dict(kind="bf16", M=8192, K=8192, N=8192, wstd=0.02, outliers=False),
 }
 DEFAULT_WORKLOAD = "fp8_groupwise_llama8b_mlp"
-# further configurations reported in `sweep` (one GPU) ...
+# further configurations, reported on stderr (one GPU) ...
 SWEEP_1GPU = ["fp8_per_tensor_1024", "fp8_groupwise_8192", "nvfp4_8192", "nvfp4_8192_static_scale", "nvfp4_8192_token_scale", "nvfp4_m1", "nvfp4_m16", "nvfp4_m128", "nvfp4_m1024",
               "mxfp4_llama70b_up", "mxfp4_llama70b_down", "moe_nvfp4", "moe_nvfp4_token_scale", "moe_nvfp4_tokens", "moe_nvfp4_skewed",
               "moe_fp8_groupwise", "moe_fp8_groupwise_tokens", "moe_layer_nvfp4"]
@@ -805,6 +805,18 @@ def host_cost_us(wl, n=200):
     return min(best)
 
 
+def one_line(record) -> str:
+    """The result as one JSON line of at most a few thousand characters (readers that keep the end of a program's output still
+    have all of it): numbers to seven digits, no sweep."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.7g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        return [short(x) for x in v] if isinstance(v, (list, tuple)) else v
+    return json.dumps(short(record))
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -816,7 +828,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-sweep", action="store_true", help="only the headline workload")
     ap.add_argument("--sweep-limit", type=float, default=420.0,
-                    help="seconds after which the line is printed with the sweep entries measured so far")
+                    help="seconds after which the line is printed although the sweep has not finished")
     ap.add_argument("--min-seconds", type=float, default=1.0, help="the K-step block is repeated until the timed region is this long")
     ap.add_argument("--scaling", default="strong", choices=["weak", "strong"],
                     help="strong (default): the one problem is split across the ranks (columns / experts); "
@@ -857,8 +869,8 @@ def main():
     del wl
     torch.cuda.empty_cache()
 
-    # The headline line is complete here; the sweep only adds to it.  A watchdog guarantees that the line is printed
-    # (and every rank exits) even if a sweep entry fails on one rank and leaves the others waiting in a collective.
+    # The line is complete here; the sweep's records go to stderr as they are measured.  A watchdog guarantees that the line is
+    # printed (and every rank exits) even if a sweep entry fails on one rank and leaves the others waiting in a collective.
     line = None
     if rank == 0:
         line = {
@@ -888,15 +900,13 @@ def main():
             if rc is not None:
                 line["reference_cuda"] = rc
 
-    sweep = []
     printed = threading.Lock()
 
     def give_up():
         if printed.acquire(blocking=False):
             if line is not None:
-                line["sweep"] = sweep
-                line["sweep_error"] = f"the sweep did not finish within {args.sweep_limit:.0f} s; entries measured so far are kept"
-                print(json.dumps(line), flush=True)
+                line["sweep_error"] = f"the sweep did not finish within {args.sweep_limit:.0f} s"
+                print(one_line(line), flush=True)
             os._exit(0)
 
     if not args.no_sweep and args.workload == DEFAULT_WORKLOAD:
@@ -913,16 +923,15 @@ def main():
                               2 if big else args.sets, False)
             except Exception as exc:     # a sweep entry must not take the headline down with it
                 rec = {"workload": name, "error": f"{type(exc).__name__}: {exc}"}
-            sweep.append(rec)
+            if rank == 0:
+                print(json.dumps(rec), file=sys.stderr, flush=True)
         watchdog.cancel()
     if not printed.acquire(blocking=False):
         return                                    # the watchdog is printing / has printed
     if sampler is not None:
         sampler.stop()
     if rank == 0:
-        if sweep:
-            line["sweep"] = sweep
-        print(json.dumps(line), flush=True)
+        print(one_line(line), flush=True)
     if dist is not None:
         dist.destroy_process_group()
 
