@@ -192,25 +192,29 @@ def _experts_fp4(p: MoEPlan, packed: torch.Tensor, sf: torch.Tensor, gs, w: MoEW
                               global_scale_b=w.down.global_scale, out_dtype=torch.bfloat16, **common)
 
 
-def _plain(t: Optional[torch.Tensor], device: torch.device, dtypes) -> bool:
-    return t is not None and t.dtype in dtypes and t.device == device and t.is_contiguous()
-
-
 def _as_packed(w: PackedWeight, device: torch.device) -> bool:
     """Whether the weight's tensors are what pack_weight makes for its format and sizes.  The one-call layer reads them by
-    pointer; anything else (assembled by hand) takes the step-by-step form, which checks or converts them."""
-    rows, q = w.groups * w.n, w.q
-    if w.format == "bf16":
-        return _plain(q, device, (torch.bfloat16,)) and q.shape == (rows, w.k)
-    fp4 = w.format in ("nvfp4", "mxfp4")
-    if not _plain(q, device, _BYTE_DTYPES) or q.shape != (rows, w.k // 2 if fp4 else w.k):
+    pointer; anything else (assembled by hand) takes the step-by-step form, which checks or converts them.  In line and in
+    this order because a layer of one token is bound by host time."""
+    q, scale, fmt = w.q, w.scale, w.format
+    rows, k = w.groups * w.n, w.k
+    if q.device != device or not q.is_contiguous():
+        return False
+    if fmt == "bf16":
+        return q.dtype is torch.bfloat16 and q.shape == (rows, k)
+    if q.dtype not in _BYTE_DTYPES or scale is None or scale.device != device or not scale.is_contiguous():
         return False
     tiles = w.groups * ((w.n + 127) // 128)
-    if not fp4:
-        return _plain(w.scale, device, (torch.float32,)) and w.scale.numel() == (1 if w.format == "fp8" else tiles * ((w.k + 127) // 128))
-    katoms = (w.k // (16 if w.format == "nvfp4" else 32) + 3) // 4
-    return (_plain(w.scale, device, _BYTE_DTYPES) and w.scale.numel() >= tiles * katoms * 512
-            and (w.format == "mxfp4" or (_plain(w.global_scale, device, (torch.float32,)) and w.global_scale.numel() == 1)))
+    if fmt == "fp8" or fmt == "fp8_block128":
+        return (q.shape == (rows, k) and scale.dtype is torch.float32
+                and scale.numel() == (1 if fmt == "fp8" else tiles * ((k + 127) // 128)))
+    if q.shape != (rows, k // 2) or scale.dtype not in _BYTE_DTYPES:
+        return False
+    if fmt == "mxfp4":
+        return scale.numel() >= tiles * ((k // 32 + 3) // 4) * 512
+    gs = w.global_scale
+    return (scale.numel() >= tiles * ((k // 16 + 3) // 4) * 512
+            and gs is not None and gs.dtype is torch.float32 and gs.device == device and gs.numel() == 1)
 
 
 def _whole_layer(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, renormalize: bool, out_dtype,
@@ -229,7 +233,7 @@ def _whole_layer(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, r
     fused = gu.format == "nvfp4" and hgs is not None
     if (fused and (isinstance(hgs, torch.Tensor) or not hgs > 0)) or isinstance(act_global_scale, str):
         return None
-    dev = _lib.require_cuda(x, logits, gu.q, dn.q)
+    dev = _lib.require_cuda(x, logits)           # the weights are on x's device
     lib = _lib.lib()
     x = x.to(torch.bfloat16).contiguous() if gu.format == "bf16" else x.contiguous()
     logits = logits.contiguous()
@@ -242,13 +246,19 @@ def _whole_layer(x: torch.Tensor, logits: torch.Tensor, w: MoEWeights, k: int, r
     need = int(lib.dsl_moe_layer_scratch_bytes(ctypes.byref(du), ctypes.byref(dd), T, k, 1 if fused else 0))
     if need == 0:
         return None
-    with torch.cuda.device(dev):
+    prev = torch.cuda.current_device()
+    if prev != dev.index:
+        torch.cuda.set_device(dev)
+    try:
         scratch = torch.empty(need, dtype=torch.uint8, device=dev)
         out = torch.empty((T, dn.n), dtype=out_dtype, device=dev)
         rc = lib.dsl_moe_layer(x.data_ptr(), _lib.dtype_code(x.dtype), logits.data_ptr(), _lib.dtype_code(logits.dtype), T, k,
                                1 if renormalize else 0, ctypes.byref(du), ctypes.byref(dd), _lib.ptr(act_gs), 1 if fused else 0,
                                float(hgs) if fused else 1.0, scratch.data_ptr(), need, out.data_ptr(), _lib.dtype_code(out_dtype),
                                _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+    finally:
+        if prev != dev.index:
+            torch.cuda.set_device(prev)
     _lib.check(rc, "dsl_moe_layer")
     return out
 
