@@ -6,8 +6,9 @@
 // so their tensor-core time is that of a full batch and they read the weight at 4.6 TB/s; here the operand roles are swapped
 // as in gemm_decode.cu: 128 weight rows (output columns) are the M side of tcgen05.mma and TOK = 32 or 64 of the group's
 // rows the N side, which leaves the tensor core mostly idle and the ring of TMA loads (7-8 stages of 16 KB of weight) to set
-// the pace.  There are more (group, column tile) pairs than SMs, so K is not cut: a CTA takes whole tiles, round robin, and
-// its ring runs on from one tile into the next.  64 experts of 3072 x 4096 NVFP4, eight rows each: 77 us = 5.9 TB/s of weight
+// the pace.  There are usually more (group, column tile) pairs than SMs, so K is not cut: a CTA takes whole tiles, round robin,
+// and its ring runs on from one tile into the next (with fewer pairs it is still ahead of the tiled kernels: 8 groups of 512
+// columns, K = 4096, 8 rows each, call with quantiser, NVFP4 23 / 31 us, BF16 26 / 28 us).  64 experts of 3072 x 4096 NVFP4, eight rows each: 77 us = 5.9 TB/s of weight
 // and scales (98 us, 4.6 TB/s, on the tiled kernel).  A group with more than TOK rows is several items on the same weight tile,
 // neighbours in the order, so that all but the first find it in the L2.
 //
@@ -419,6 +420,15 @@ static int launch_grouped_kind(const void* A, const void* B, const GemmArgs& arg
 //   FP8 per tensor     243 / 285    249 / 293    261 / 301    267 / 343
 //   BF16               418 / 489    442 / 508    445 / 519    431 / 660
 // and with one row for each of eight experts 72 / 76, 79 / 92, 87 / 99, 99 / 136.
+// The sizes of the groups are on the device, so the rule sees their mean only.  Skewed groups, the gate/up GEMM of that layer
+// (64 groups, N = 3072, K = 4096, quantiser included, L2 cold; this kernel / the tiled kernels, us):
+//                       512 rows:  even       all in 8   all in 1 | 2048 rows: even     half in 1  0.9 in 1   all in 8  all in 1
+//   NVFP4                        111 / 122   41 / 49    38 / 42   |          123 / 136  134 / 140  145 / 142  76 / 66   76 / 62
+//   FP8 128x128 blocks           149 / 230   44 / 54    42 / 34   |          173 / 239  194 / 245  224 / 249 114 / 60  112 / 56
+//   FP8 per tensor               154 / 172   49 / 53    45 / 37   |          170 / 187  181 / 193  197 / 193  88 / 73   86 / 67
+//   BF16                         267 / 308   65 / 73    58 / 36   |          273 / 321  300 / 329  331 / 323 114 / 79  112 / 60
+// While the weights of most groups are read this kernel is ahead or even; it falls behind, to half the speed, only where nearly
+// all rows sit in a few groups, whose weight the taller tiles of the other kernels read fewer times.
 constexpr int kGroupedMeanRows = 32;
 
 bool decode_grouped_served(const GemmArgs& args) {
