@@ -21,7 +21,9 @@ namespace dsl {
 // with programmatic stream serialisation: a step's CTAs are placed while the step before it still runs and wait here, before
 // they touch any memory, until it has completed.  A step lets its own successor start only after that wait, so that when a
 // kernel of the chain starts, everything before its predecessor is complete: a successor that fetches a weight early
-// (dsl_epilogue.b_is_static) relies on it.
+// (dsl_epilogue.b_is_static) relies on it.  Layer of 64 experts, top 8, K = D = 4096, H = 1536, the same weights call after call,
+// launched the plain way (GEMMs too) / so: NVFP4 one token 74 / 70 us, 8 tokens 129 / 117, 64 165 / 147, 512 223 / 206; FP8 128x128
+// blocks 64 tokens 241 / 227.
 __device__ __forceinline__ void chain_link() {
     griddep_wait();
     griddep_launch_dependents();

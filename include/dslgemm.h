@@ -132,8 +132,10 @@ typedef struct {
     void* workspace;            /* optional scratch (16-byte aligned) for partial sums along K, or NULL */
     size_t workspace_bytes;     /* its size: dsl_workspace_bytes() says what a problem can put to use (less is
                                    allowed and only slower).  The first 64 KiB are a header in which only the
-                                   weight-streaming kernel's arrival words ever live; the buffer need not be cleared,
-                                   and launches that may overlap on the GPU need separate buffers */
+                                   weight-streaming kernel's arrival words ever live; the buffer need not be cleared.
+                                   A call may leave sums here for its own next launch: calls that may overlap on the
+                                   GPU, and host threads that issue calls on one stream at the same time, need
+                                   separate buffers */
     int b_is_static;            /* non-zero: B and its scale bytes are not written by the kernel that precedes this
                                    call in the stream (a pre-packed weight).  The weight-streaming kernel is launched
                                    with programmatic stream serialisation and then starts fetching B while that
